@@ -1,6 +1,7 @@
 // C ABI of the diskgpu library (include/diskgpu.h): handle life cycle, state transfer,
 // and the device-resident step loop.  The kernels live in kernels64.cu (plain FP64 path)
 // and mixed*.cu (FP32 perturbation + tensor-core gravity).
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -35,10 +36,11 @@ int dg_handle::fail(int code, const char *what, const char *why) {
   return code;
 }
 
-static std::vector<double2> roots_table(int n) {
+// e^{-2 pi i j / M}, j < n
+static std::vector<double2> roots_table(int n, int M) {
   std::vector<double2> r(n);
   for (int t = 0; t < n; ++t) {
-    long double a = 2.0L * 3.141592653589793238462643383279502884L * (long double)t / (long double)n;
+    long double a = 2.0L * 3.141592653589793238462643383279502884L * (long double)t / (long double)M;
     r[t].x = (double)cosl(a);
     r[t].y = (double)-sinl(a);
   }
@@ -56,7 +58,7 @@ static cudaError_t dmalloc(T **p, size_t n) {
 static int validate(const dg_params *p, std::string *why) {
   char b[256];
   if (p->Nu < 2 || p->Nphi < 2) { snprintf(b, sizeof b, "Nu=%d Nphi=%d: both must be >= 2", p->Nu, p->Nphi); *why = b; return DG_ERR_INVALID; }
-  // one CTA holds a whole transform (<= 8192 points: 1024 threads x 8, 128 KiB of FP64 complex)
+  // one CTA holds a whole transform: 8192 points of FP64 complex in phi, two of 4096 in u
   if (p->Nu > 4096 || p->Nphi > 8192) { snprintf(b, sizeof b, "Nu=%d Nphi=%d exceeds 4096 x 8192", p->Nu, p->Nphi); *why = b; return DG_ERR_UNSUPPORTED; }
   if (!(p->Rin > 0) || !(p->Rout > p->Rin)) { *why = "need 0 < Rin < Rout"; return DG_ERR_INVALID; }
   if (!(p->Kpoly > 0) || !(p->gamma_gas > 0)) { *why = "need Kpoly > 0 and gamma_gas > 0"; return DG_ERR_INVALID; }
@@ -64,7 +66,7 @@ static int validate(const dg_params *p, std::string *why) {
   if (p->precision != DG_PREC_FP64 && p->precision != DG_PREC_MIXED) { *why = "precision must be DG_PREC_FP64 or DG_PREC_MIXED"; return DG_ERR_INVALID; }
   if (p->basic_state != DG_BASIC_FFT && p->basic_state != DG_BASIC_ELLIPTIC) { *why = "basic_state must be DG_BASIC_FFT or DG_BASIC_ELLIPTIC"; return DG_ERR_INVALID; }
   FftPlan a, c;
-  if (!make_fft_plan(p->Nphi, &a) || !make_fft_plan(2 * p->Nu, &c)) {
+  if (!make_fft_plan(p->Nphi, &a) || !make_fft_plan(p->Nu, &c)) {
     snprintf(b, sizeof b, "Nphi=%d and 2*Nu=%d must factor into 2, 3 and 5", p->Nphi, 2 * p->Nu);
     *why = b;
     return DG_ERR_UNSUPPORTED;
@@ -95,7 +97,7 @@ int dg_handle::init(const dg_params &pp) {
   M = 2 * Nu;
   Nc = Nphi / 2 + 1;
   make_fft_plan(Nphi, &plPhi);
-  make_fft_plan(M, &plM);
+  make_fft_plan(Nu, &plU);
   const size_t n = (size_t)Nu * Nphi;
   MK(dmalloc(&dR, Nu)); MK(dmalloc(&dRf, Nu + 1)); MK(dmalloc(&dVol, Nu));
   MK(dmalloc(&dSqrtR, Nu)); MK(dmalloc(&dR32, Nu));
@@ -111,11 +113,29 @@ int dg_handle::init(const dg_params &pp) {
     MK(cudaMemset(VP[b], 0, n * sizeof(double)));
   }
   MK(dmalloc(&dPhi, n)); MK(dmalloc(&gA, n)); MK(dmalloc(&gB, n));
-  MK(dmalloc(&W, (size_t)Nc * M)); MK(dmalloc(&Khat, (size_t)Nc * M));
-  std::vector<double2> r1 = roots_table(Nphi), r2 = roots_table(M);
-  MK(dmalloc(&rootsPhi, Nphi)); MK(dmalloc(&rootsM, M));
-  MK(cudaMemcpy(rootsPhi, r1.data(), Nphi * sizeof(double2), cudaMemcpyHostToDevice));
-  MK(cudaMemcpy(rootsM, r2.data(), M * sizeof(double2), cudaMemcpyHostToDevice));
+  ldW = Nu + (Nu & 1);
+  MK(dmalloc(&W, (size_t)Nc * ldW)); MK(dmalloc(&Khat, (size_t)Nc * M));
+  {
+    // one buffer: stage twiddles of both directions, e^{-2 pi i j / M}, then the positions
+    std::vector<double2> t1, t2, hf = roots_table(Nu, M);
+    std::vector<unsigned short> p1, p2;
+    fft_tables(plPhi, &t1, &p1);
+    fft_tables(plU, &t2, &p2);
+    const size_t n1 = t1.size(), n2 = t2.size(), npos = ((size_t)Nphi + Nu + 7) / 8;
+    std::vector<double2> t(n1 + n2 + Nu + npos);
+    std::copy(t1.begin(), t1.end(), t.begin());
+    std::copy(t2.begin(), t2.end(), t.begin() + n1);
+    std::copy(hf.begin(), hf.end(), t.begin() + n1 + n2);
+    unsigned short *ps = reinterpret_cast<unsigned short *>(t.data() + n1 + n2 + Nu);
+    std::copy(p1.begin(), p1.end(), ps);
+    std::copy(p2.begin(), p2.end(), ps + Nphi);
+    MK(dmalloc(&twPhi, t.size()));
+    MK(cudaMemcpy(twPhi, t.data(), t.size() * sizeof(double2), cudaMemcpyHostToDevice));
+    twU = twPhi + n1;
+    halfU = twU + n2;
+    posPhi = reinterpret_cast<unsigned short *>(halfU + Nu);
+    posU = posPhi + Nphi;
+  }
   MK(dmalloc(&scratch, 64));
   MK(dmalloc(&ctl, 1));
   MK(cudaMemset(ctl, 0, sizeof(Ctl)));
@@ -161,13 +181,16 @@ int dg_handle::init(const dg_params &pp) {
 
 // kalnajs.hpp:105-116: khat = r2c of the kernel sampled at wrapped offsets.
 int dg_handle::build_khat() {
-  double *tmp = nullptr;
-  MK(dmalloc(&tmp, (size_t)M * p.Nphi));
-  MK(launch_kernel_samples64(tmp, M, p.Nphi, du, dphi, p.eps, st));
-  MK(launch_phi_fwd<double>(tmp, M, p.Nphi, nullptr, W, M, plPhi, rootsPhi, st));
-  MK(launch_u_conv<double>(W, M, Nc, M, M, plM, rootsM, nullptr, Khat, st));
-  MK(cudaStreamSynchronize(st));
-  MK(cudaFree(tmp));
+  const size_t ns = (size_t)M * p.Nphi;
+  double2 *spec = nullptr;  // the samples' phi spectra [m][p], then the samples
+  MK(dmalloc(&spec, (size_t)Nc * M + (ns + 1) / 2));
+  double *tmp = reinterpret_cast<double *>(spec + (size_t)Nc * M);
+  cudaError_t e = launch_kernel_samples64(tmp, M, p.Nphi, du, dphi, p.eps, st);
+  if (e == cudaSuccess) e = launch_phi_fwd(tmp, M, nullptr, spec, M, plPhi, twPhi, posPhi, st);
+  if (e == cudaSuccess) e = launch_u_khat(spec, M, Nc, plU, twU, halfU, Khat, st);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  cudaFree(spec);
+  MK(e);
   return DG_OK;
 }
 
@@ -178,7 +201,7 @@ void dg_handle::release() {
   if (graph_exec) cudaGraphExecDestroy(graph_exec);
   if (diag) cudaFree(diag);
   void *ptrs[] = {rowtab, dR, dRf, dVol, dSqrtR, dR32, S[0], S[1], VR[0], VR[1], VP[0], VP[1], dPhi, gA, gB,
-                  W, Khat, rootsPhi, rootsM, scratch, ctl};
+                  W, Khat, twPhi, scratch, ctl};
   for (void *q : ptrs)
     if (q) cudaFree(q);
   if (hctl) cudaFreeHost(hctl);
@@ -191,14 +214,14 @@ void dg_handle::release() {
 // gravity (FP64): kalnajs.hpp:48-63
 int dg_handle::potential64(const double *dSig, double *dOut) {
   MK(prof_begin(DG_PROF_GRAV_PHI_FWD));
-  MK(launch_phi_fwd<double>(dSig, p.Nu, p.Nphi, dR32, W, M, plPhi, rootsPhi, st));
+  MK(launch_phi_fwd(dSig, p.Nu, dR32, W, ldW, plPhi, twPhi, posPhi, st));
   MK(prof_end(DG_PROF_GRAV_PHI_FWD));
   MK(prof_begin(DG_PROF_GRAV_U));
-  MK(launch_u_conv<double>(W, M, Nc, p.Nu, p.Nu, plM, rootsM, Khat, nullptr, st));
+  MK(launch_u_conv(W, ldW, Nc, plU, twU, halfU, Khat, st));
   MK(prof_end(DG_PROF_GRAV_U));
   const double pref = -p.G * du * dphi / (static_cast<double>(M) * p.Nphi);
   MK(prof_begin(DG_PROF_GRAV_PHI_INV));
-  MK(launch_phi_inv<double>(W, M, p.Nu, p.Nphi, plPhi, rootsPhi, pref, dSqrtR, dOut, st));
+  MK(launch_phi_inv(W, ldW, p.Nu, plPhi, twPhi, posPhi, pref, dSqrtR, dOut, st));
   MK(prof_end(DG_PROF_GRAV_PHI_INV));
   return DG_OK;
 }

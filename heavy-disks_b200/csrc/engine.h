@@ -40,8 +40,15 @@ struct dg_handle {
   double *S[2] = {nullptr, nullptr}, *VR[2] = {nullptr, nullptr}, *VP[2] = {nullptr, nullptr};
   int cur = 0;
   double *dPhi = nullptr, *gA = nullptr, *gB = nullptr;
-  double2 *W = nullptr, *Khat = nullptr, *rootsPhi = nullptr, *rootsM = nullptr;
-  dg::FftPlan plPhi{}, plM{};
+  // phi half spectra [m][i], row stride ldW (Nu rounded up to even); the real khat table
+  // (fft_smem.cuh k_u_khat, read through
+  // khat_at); stage twiddles, e^{-2 pi i j / 2 Nu} and
+  // frequency positions of the transforms (one buffer, owned by twPhi)
+  double2 *W = nullptr, *twPhi = nullptr, *twU = nullptr, *halfU = nullptr;
+  double *Khat = nullptr;
+  int ldW = 0;
+  unsigned short *posPhi = nullptr, *posU = nullptr;
+  dg::FftPlan plPhi{}, plU{};
   double *scratch = nullptr;  // 64 doubles of reduction output
 
   // control block (device) and a pinned host mirror

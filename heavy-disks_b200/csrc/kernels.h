@@ -3,9 +3,12 @@
 
 #include <cuda_runtime.h>
 
+#include <utility>
+#include <vector>
+
 #include "dg_common.cuh"
 #include "hydro64.cuh"
-#include "fft_smem.cuh"
+#include "fft_plan.cuh"
 
 namespace dg {
 
@@ -21,17 +24,34 @@ cudaError_t launch_conserved64(const double *Sig, const double *vp, const Geom64
 cudaError_t launch_kernel_samples64(double *out, int M, int Nphi, double du, double dphi, double eps,
                                     cudaStream_t st);
 
+// Launch with programmatic stream serialization: the kernel may begin (its prologue up to
+// pdl_wait) while the previous kernel on the stream drains.
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                              Args &&...args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
+}
+
 bool make_fft_plan(int n, FftPlan *pl);
+void fft_tables(const FftPlan &pl, std::vector<double2> *tw, std::vector<unsigned short> *pos);
 cudaError_t prepare_fft_kernels();
-template <typename T>
-cudaError_t launch_phi_fwd(const T *src, int nrows, int Nphi, const T *rowscale, typename cplx_of<T>::type *W,
-                           int ldw, const FftPlan &pl, const typename cplx_of<T>::type *roots, cudaStream_t st);
-template <typename T>
-cudaError_t launch_u_conv(typename cplx_of<T>::type *W, int ldw, int Nc, int nin, int nout, const FftPlan &pl,
-                          const typename cplx_of<T>::type *roots, const typename cplx_of<T>::type *khat,
-                          typename cplx_of<T>::type *kout, cudaStream_t st);
-template <typename T>
-cudaError_t launch_phi_inv(const typename cplx_of<T>::type *W, int ldw, int nrows, int Nphi, const FftPlan &pl,
-                           const typename cplx_of<T>::type *roots, T pref, const T *sqrtR, T *out, cudaStream_t st);
+cudaError_t launch_phi_fwd(const double *src, int nrows, const double *rowscale, double2 *W, int ldw,
+                           const FftPlan &pl, const double2 *tws, const unsigned short *pos, cudaStream_t st);
+cudaError_t launch_u_conv(double2 *W, int ldw, int Nc, const FftPlan &pl, const double2 *tws, const double2 *half,
+                          const double *kr, cudaStream_t st);
+cudaError_t launch_u_khat(const double2 *W, int ldw, int Nc, const FftPlan &pl, const double2 *tws, const double2 *half,
+                          double *kr, cudaStream_t st);
+cudaError_t launch_phi_inv(const double2 *W, int ldw, int nrows, const FftPlan &pl, const double2 *tws,
+                           const unsigned short *pos, double pref, const double *sqrtR, double *out, cudaStream_t st);
 
 }  // namespace dg

@@ -1,5 +1,7 @@
 // Plain-method (FP64) kernels: fused hydro step, CFL reduction, forces, mode sums,
 // Kalnajs kernel samples, and launchers for the shared-memory FFT passes.
+#include <cmath>
+
 #include "kernels.h"
 #include "hydro64.cuh"
 #include "fft_smem.cuh"
@@ -415,42 +417,75 @@ cudaError_t launch_kernel_samples64(double *out, int M, int Nphi, double du, dou
 }
 
 // ---------------------------------------------------------------------------------
-// FFT pass launchers.  Each picks (E, nb, threads) with nb * n <= E * threads.
+// FFT plans and pass launchers.
+
+// Stage radices: the factors 5 and 3 first, then the power of two in radices 8 and 4.  Radix
+// 16 would save a stage of some lengths, but its registers halve the warps per SM, and a
+// stage costs less than the latency those warps hide.
 bool make_fft_plan(int n, FftPlan *pl) {
+  *pl = FftPlan{};
+  if (n < 1) return false;
   pl->n = n;
-  pl->n4 = pl->n2 = pl->n3 = pl->n5 = 0;
-  int m = n;
-  while (m % 4 == 0) { pl->n4++; m /= 4; }
-  while (m % 2 == 0) { pl->n2++; m /= 2; }
-  while (m % 3 == 0) { pl->n3++; m /= 3; }
-  while (m % 5 == 0) { pl->n5++; m /= 5; }
-  return m == 1 && n >= 1;
-}
-
-struct FftShape {
-  int E, nb, threads;
-  size_t smem;
-};
-
-template <typename V>
-static FftShape fft_shape(int n, int count) {
-  // Prefer 256 threads and 8 elements per thread; shrink nb to fill >= 2 waves of SMs.
-  FftShape s;
-  s.E = 8;
-  s.threads = 256;
-  if (n > s.E * s.threads) {
-    s.threads = (n + s.E - 1) / s.E;
-    s.threads = ((s.threads + 31) / 32) * 32;
-    if (s.threads > 1024) s.threads = 1024;  // n <= 8192
+  int e = 0, rest = n;
+  while (rest % 2 == 0) { ++e; rest /= 2; }
+  auto add = [&](int R) { pl->R[pl->ns++] = R; };
+  while (rest % 5 == 0) { add(5); rest /= 5; }
+  while (rest % 3 == 0) { add(3); rest /= 3; }
+  if (rest != 1) return false;
+  while (e > 0) {
+    const int k = (e <= 3) ? e : (e == 4 ? 2 : 3);
+    add(1 << k);
+    e -= k;
   }
-  s.nb = (s.E * s.threads) / n;
-  if (s.nb < 1) s.nb = 1;
-  int want = 2 * sm_count();
-  while (s.nb > 1 && (count + s.nb - 1) / s.nb < want) s.nb /= 2;
-  s.smem = (size_t)s.nb * n * sizeof(V);
-  return s;
+  if (pl->ns == 0) return false;  // n = 1
+  int L = n;
+  for (int s = 0; s < pl->ns; ++s) {
+    const int R = pl->R[s], m = L / R;
+    pl->m[s] = m;
+    pl->magic[s] = m > 1 ? (unsigned)(((1ull << 32) + m - 1) / m) : 0u;
+    pl->tw[s] = pl->ntw;
+    pl->ntw += (R - 1) * m;
+    L = m;
+  }
+  // threads per transform: one butterfly each in a radix-8 stage of a long transform; a
+  // short one, whose few CTAs leave the SMs idle anyway, takes more for its loads and stores
+  // (FP64 step at 64^2 / 128^2: 19.5 / 21.2 us with n / 4 threads, 18.6 / 20.5 with n / 2;
+  // at 512^2 34.9 us with n / 4, 32.7 with n / 8)
+  int T = n >= 512 ? (n + 7) / 8 : (n + 1) / 2;
+  if (T > kFftMaxThreads / 2) T = kFftMaxThreads / 2;
+  pl->threads = T < 1 ? 1 : T;
+  return true;
 }
 
+// Host tables of a plan: the stage twiddles and the position of every frequency.
+void fft_tables(const FftPlan &pl, std::vector<double2> *tw, std::vector<unsigned short> *pos) {
+  tw->assign(pl.ntw, make_double2(1.0, 0.0));
+  for (int s = 0; s < pl.ns; ++s) {
+    const int R = pl.R[s], m = pl.m[s], L = R * m;
+    for (int q = 1; q < R; ++q)
+      for (int j = 0; j < m; ++j) {
+        const long double a = -2.0L * 3.141592653589793238462643383279502884L * (long double)(j * q) / (long double)L;
+        (*tw)[pl.tw[s] + (q - 1) * m + j] = make_double2((double)cosl(a), (double)sinl(a));
+      }
+  }
+  pos->assign(pl.n, 0);
+  for (int k = 0; k < pl.n; ++k) {  // k = q0 + R0 (q1 + R1 (...)) sits at q0 m0 + q1 m1 + ...
+    int r = k, at = 0;
+    for (int s = 0; s < pl.ns; ++s) {
+      at += (r % pl.R[s]) * pl.m[s];
+      r /= pl.R[s];
+    }
+    (*pos)[k] = (unsigned short)at;
+  }
+}
+
+// Transforms per CTA: up to 4 (their rows share the 128-byte runs of W), while every SM
+// still gets a CTA.
+static int fft_log2_batch(const FftPlan &pl, int count) {
+  int lg = 0;
+  while (lg < 2 && (pl.threads << (lg + 1)) <= kFftMaxThreads && (count >> (lg + 1)) >= sm_count()) ++lg;
+  return lg;
+}
 
 // Raise the dynamic shared-memory limit of every FFT pass once, outside any graph capture.
 cudaError_t prepare_fft_kernels() {
@@ -459,8 +494,9 @@ cudaError_t prepare_fft_kernels() {
   int dev = 0, optin = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-  const void *fns[] = {(const void *)k_phi_fwd<double, 8>, (const void *)k_u_conv<double, 8>,
-                       (const void *)k_phi_inv<double, 8>};
+  const void *fns[] = {(const void *)k_phi_fwd<true>, (const void *)k_phi_fwd<false>, (const void *)k_u_conv<true>,
+                       (const void *)k_u_conv<false>, (const void *)k_u_khat, (const void *)k_phi_inv<true>,
+                       (const void *)k_phi_inv<false>};
   for (const void *f : fns) {
     cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
     if (e != cudaSuccess) return e;
@@ -469,48 +505,39 @@ cudaError_t prepare_fft_kernels() {
   return cudaSuccess;
 }
 
-template <typename T>
-cudaError_t launch_phi_fwd(const T *src, int nrows, int Nphi, const T *rowscale, typename cplx_of<T>::type *W,
-                           int ldw, const FftPlan &pl, const typename cplx_of<T>::type *roots, cudaStream_t st) {
-  using V = typename cplx_of<T>::type;
-  FftShape s = fft_shape<V>(Nphi, (nrows + 1) / 2);
-  int blocks = (nrows + 2 * s.nb - 1) / (2 * s.nb);
-  {
-    k_phi_fwd<T, 8><<<blocks, s.threads, s.smem, st>>>(src, nrows, Nphi, rowscale, W, ldw, pl, roots, s.nb);
-  }
+// Lengths whose tables go to shared memory (the SMT forms).
+static bool fft_smt(int n) { return n <= 512; }
+
+cudaError_t launch_phi_fwd(const double *src, int nrows, const double *rowscale, double2 *W, int ldw,
+                           const FftPlan &pl, const double2 *tws, const unsigned short *pos, cudaStream_t st) {
+  const int pairs = (nrows + 1) / 2, lg = fft_log2_batch(pl, pairs), nb = 1 << lg;
+  const bool smt = fft_smt(pl.n);
+  const size_t sm = ((size_t)nb * fft_pad_len(pl.n) + (smt ? fft_tab_phi(pl.n, pl.ntw) : 0)) * sizeof(double2);
+  return launch_pdl(smt ? k_phi_fwd<true> : k_phi_fwd<false>, dim3((pairs + nb - 1) / nb), dim3(pl.threads, nb), sm,
+                    st, src, nrows, rowscale, W, ldw, pl, tws, pos, lg);
+}
+
+cudaError_t launch_u_conv(double2 *W, int ldw, int Nc, const FftPlan &pl, const double2 *tws, const double2 *half,
+                          const double *kr, cudaStream_t st) {
+  const bool smt = fft_smt(pl.n);
+  const size_t sm = ((size_t)2 * fft_pad_len(pl.n) + (smt ? fft_tab_u(pl.n, pl.ntw) : 0)) * sizeof(double2);
+  return launch_pdl(smt ? k_u_conv<true> : k_u_conv<false>, dim3(Nc), dim3(pl.threads, 2), sm, st, W, ldw, pl, tws,
+                    half, kr);
+}
+
+cudaError_t launch_u_khat(const double2 *W, int ldw, int Nc, const FftPlan &pl, const double2 *tws, const double2 *half,
+                          double *kr, cudaStream_t st) {
+  k_u_khat<<<2 * Nc, pl.threads, (size_t)fft_pad_len(pl.n) * sizeof(double2), st>>>(W, ldw, pl, tws, half, kr);
   return cudaGetLastError();
 }
 
-template <typename T>
-cudaError_t launch_u_conv(typename cplx_of<T>::type *W, int ldw, int Nc, int nin, int nout, const FftPlan &pl,
-                          const typename cplx_of<T>::type *roots, const typename cplx_of<T>::type *khat,
-                          typename cplx_of<T>::type *kout, cudaStream_t st) {
-  using V = typename cplx_of<T>::type;
-  FftShape s = fft_shape<V>(pl.n, Nc);
-  int blocks = (Nc + s.nb - 1) / s.nb;
-  {
-    k_u_conv<T, 8><<<blocks, s.threads, s.smem, st>>>(W, ldw, Nc, nin, nout, pl, roots, khat, kout, s.nb);
-  }
-  return cudaGetLastError();
+cudaError_t launch_phi_inv(const double2 *W, int ldw, int nrows, const FftPlan &pl, const double2 *tws,
+                           const unsigned short *pos, double pref, const double *sqrtR, double *out, cudaStream_t st) {
+  const int pairs = (nrows + 1) / 2, lg = fft_log2_batch(pl, pairs), nb = 1 << lg;
+  const bool smt = fft_smt(pl.n);
+  const size_t sm = ((size_t)nb * fft_pad_len(pl.n) + (smt ? fft_tab_phi(pl.n, pl.ntw) : 0)) * sizeof(double2);
+  return launch_pdl(smt ? k_phi_inv<true> : k_phi_inv<false>, dim3((pairs + nb - 1) / nb), dim3(pl.threads, nb), sm,
+                    st, W, ldw, nrows, pl, tws, pos, pref, sqrtR, out, lg);
 }
-
-template <typename T>
-cudaError_t launch_phi_inv(const typename cplx_of<T>::type *W, int ldw, int nrows, int Nphi, const FftPlan &pl,
-                           const typename cplx_of<T>::type *roots, T pref, const T *sqrtR, T *out, cudaStream_t st) {
-  using V = typename cplx_of<T>::type;
-  FftShape s = fft_shape<V>(Nphi, (nrows + 1) / 2);
-  int blocks = (nrows + 2 * s.nb - 1) / (2 * s.nb);
-  {
-    k_phi_inv<T, 8><<<blocks, s.threads, s.smem, st>>>(W, ldw, nrows, Nphi, pl, roots, pref, sqrtR, out, s.nb);
-  }
-  return cudaGetLastError();
-}
-
-template cudaError_t launch_phi_fwd<double>(const double *, int, int, const double *, double2 *, int,
-                                            const FftPlan &, const double2 *, cudaStream_t);
-template cudaError_t launch_u_conv<double>(double2 *, int, int, int, int, const FftPlan &, const double2 *,
-                                           const double2 *, double2 *, cudaStream_t);
-template cudaError_t launch_phi_inv<double>(const double2 *, int, int, int, const FftPlan &, const double2 *,
-                                            double, const double *, double *, cudaStream_t);
 
 }  // namespace dg

@@ -263,8 +263,8 @@ __global__ void k_tab_u(SplitBuf Cu, SplitBuf CuT, int Nu) {
   }
 }
 
-// KW[c][p] = (w_p / M) Re khat(p, m(c)); khat is the FP64 r2c table [m][0..M)
-__global__ void k_tab_kw(float *KW, const double2 *khat, int Nu, int Nphi) {
+// KW[c][p] = (w_p / M) Re khat(p, m(c)), from the FP64 table (khat_at)
+__global__ void k_tab_kw(float *KW, const double *khat, const unsigned short *posu, int Nu, int Nphi) {
   const int M = 2 * Nu;
   const size_t n = (size_t)Nphi * M;
   for (size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x) {
@@ -273,7 +273,7 @@ __global__ void k_tab_kw(float *KW, const double2 *khat, int Nu, int Nphi) {
     phi_mode(c, Nphi, m, im);
     int pp = p > Nu ? p - Nu : p;
     double wgt = (p == 0 || p == Nu) ? 1.0 : 2.0;
-    KW[k] = (float)(wgt / M * khat[(size_t)m * M + pp].x);
+    KW[k] = (float)(wgt / M * khat_at(khat, posu, Nu, m, pp));
   }
 }
 
@@ -322,13 +322,13 @@ __global__ void k_tab_cblock(SplitBuf T, int nr, int nk, int L, int sgn) {
 }
 
 // KW2[(m, p2)][(p1, ri)] = Re khat(p2 + 64 p1, m) / M for m <= Nphi/2 (padding modes: 0)
-__global__ void k_tab_kw2(float *KW2, const double2 *khat, int nm, int A, int Nphi) {
+__global__ void k_tab_kw2(float *KW2, const double *khat, const unsigned short *posu, int nm, int A, int Nphi) {
   const int M = 64 * A;
   const size_t n = (size_t)nm * 64 * 2 * A;
   for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (size_t)gridDim.x * blockDim.x) {
     const int row = (int)(q / (2 * A)), col = (int)(q % (2 * A));
     const int m = row >> 6, p2 = row & 63, p1 = col >> 1;
-    KW2[q] = (m <= Nphi / 2) ? (float)(khat[(size_t)m * M + p2 + 64 * p1].x / M) : 0.f;
+    KW2[q] = (m <= Nphi / 2) ? (float)(khat_at(khat, posu, M / 2, m, p2 + 64 * p1) / M) : 0.f;
   }
 }
 
@@ -359,12 +359,13 @@ __global__ void k_tab_phiA(SplitBuf C) {
 
 // KHM[m][p] = Re khat(p, m) / M for m <= Nphi/2 (padding modes: 0); with real_dft_weights
 // also times w_m / Nphi (w = 1 at m = 0 and Nphi/2, else 2), the inverse real DFT's weights
-__global__ void k_tab_khm(float *KHM, const double2 *khat, int nm, int M, int Nphi, bool real_dft_weights) {
+__global__ void k_tab_khm(float *KHM, const double *khat, const unsigned short *posu, int nm, int M, int Nphi,
+                          bool real_dft_weights) {
   const size_t n = (size_t)nm * M;
   for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (size_t)gridDim.x * blockDim.x) {
     const int m = (int)(q / M);
     const double w = !real_dft_weights ? 1.0 : ((m == 0 || 2 * m == Nphi) ? 1.0 : 2.0) / Nphi;
-    KHM[q] = (m <= Nphi / 2) ? (float)(khat[q].x / M * w) : 0.f;
+    KHM[q] = (m <= Nphi / 2) ? (float)(khat_at(khat, posu, M / 2, m, (int)(q % M)) / M * w) : 0.f;
   }
 }
 
@@ -571,24 +572,6 @@ static void free_split(SplitBuf &b) {
   b.hi = b.lo = nullptr;
 }
 
-// Launch with programmatic stream serialization: the kernel may begin (its prologue up to
-// pdl_wait) while the previous kernel on the stream drains.
-template <typename... KArgs, typename... Args>
-static cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
-                              Args &&...args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = block;
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
-}
-
 // a product slot's "stages" values that select the persistent GEMM (tc_gemm.cuh), with
 // 128 x 128 or (where N is a multiple of 256) 128 x 256 tiles
 constexpr int kPersist = 8, kPersistWide = 16;
@@ -701,7 +684,7 @@ int dg_handle::mixed_init() {
   XK(cudaGetLastError());
   k_tab_u<<<grid_for((size_t)2 * Nu * Nu), 256, 0, st>>>(X.Cu, X.CuT, Nu);
   XK(cudaGetLastError());
-  k_tab_kw<<<grid_for((size_t)Nphi * 2 * Nu), 256, 0, st>>>(X.KW, Khat, Nu, Nphi);
+  k_tab_kw<<<grid_for((size_t)Nphi * 2 * Nu), 256, 0, st>>>(X.KW, Khat, posU, Nu, Nphi);
   XK(cudaGetLastError());
   std::vector<float> ps(Nu);
   for (int i = 0; i < Nu; ++i) ps[i] = (float)(-p.G * du * dphi / sqrtR[i]);
@@ -738,7 +721,7 @@ int dg_handle::mixed_init() {
     k_tab_cblock<<<64, 256, 0, st>>>(X.RA, A, A, A, -1);       // W_A^{p1 i1}
     k_tab_cblock<<<64, 256, 0, st>>>(X.RGA, A, A, A, +1);      // W_A^{-i1 p1}
     k_tab_cblock<<<64, 256, 0, st>>>(X.RGB, 32, 64, 64, +1);   // W_64^{-i2 p2}
-    k_tab_kw2<<<grid_for((size_t)nm * 128 * A), 256, 0, st>>>(X.KW2, Khat, nm, A, Nphi);
+    k_tab_kw2<<<grid_for((size_t)nm * 128 * A), 256, 0, st>>>(X.KW2, Khat, posU, nm, A, Nphi);
     k_tab_tw<<<64, 256, 0, st>>>(X.tw, A, A);
     XK(cudaGetLastError());
     X.fused_u = u_fused(Nu);
@@ -747,7 +730,7 @@ int dg_handle::mixed_init() {
       XK(dalloc(&X.khm, (size_t)nm * 64 * A));
       XK(dalloc(&X.twp, (size_t)64 * tc::kUcTwLd));
       k_tab_tw<<<64, 256, 0, st>>>(X.twp, A, tc::kUcTwLd);
-      k_tab_khm<<<grid_for((size_t)nm * 64 * A), 256, 0, st>>>(X.khm, Khat, nm, 64 * A, Nphi, X.fused_phi);
+      k_tab_khm<<<grid_for((size_t)nm * 64 * A), 256, 0, st>>>(X.khm, Khat, posU, nm, 64 * A, Nphi, X.fused_phi);
       XK(cudaGetLastError());
       XK(smem_attrs((const void *)tc::k_uconv, tc::kUcSmem));
     }
