@@ -143,30 +143,39 @@ int dg_handle::init(const dg_params &pp) {
   memset(hctl, 0, sizeof(Ctl));
   MK(cudaMallocHost((void **)&hdt, sizeof(double)));
   {
-    // per-row / per-face FP64 constants of the hydro kernel
-    std::vector<double> t((size_t)8 * (Nu + 1), 0.0);
-    auto col = [&](int k) { return t.data() + (size_t)k * (Nu + 1); };
+    // per-row / per-face FP64 constants of the hydro kernel, and the CFL columns
+    std::vector<double> t((size_t)kRow64W * (Nu + 1) + 2 * (size_t)Nu, 0.0);
+    double *cR = t.data() + (size_t)kRow64W * (Nu + 1), *cl = cR + Nu;
     for (int i = 0; i < Nu; ++i) {
-      int im = i - 1 > 0 ? i - 1 : 0, ip = i + 1 < Nu - 1 ? i + 1 : Nu - 1;
-      col(0)[i] = -p.gmstar / (R[i] * R[i]);
-      col(1)[i] = 1.0 / R[i];
-      col(2)[i] = 1.0 / (R[ip] - R[im]);
-      col(3)[i] = 1.0 / Vol[i];
-      col(4)[i] = 1.0 / (Rf[i + 1] - Rf[i]);
-      col(5)[i] = 1.0 / (R[i] * dphi);
+      double *c = t.data() + (size_t)kRow64W * i;
+      const int im = i - 1 > 0 ? i - 1 : 0, ip = i + 1 < Nu - 1 ? i + 1 : Nu - 1;
+      c[hGstar] = -p.gmstar / (R[i] * R[i]);
+      c[hInvR] = 1.0 / R[i];
+      c[hInvdRc] = 1.0 / (R[ip] - R[im]);
+      c[hPhiu] = -1.0 / ((i == 0 || i == Nu - 1 ? du : 2.0 * du) * R[i]);
+      c[hPhip] = -1.0 / (2.0 * dphi * R[i]);
+      c[hCvol] = 1.0 / Vol[i];
+      c[hAphi] = Rf[i + 1] - Rf[i];
+      c[hCphi] = 0.5 / (R[i] * dphi);
+      cR[i] = c[hInvdR] = 1.0 / (Rf[i + 1] - Rf[i]);
+      cl[i] = c[hInvdl] = 1.0 / (R[i] * dphi);
+      c[hDA] = R[i] * (Rf[i + 1] - Rf[i]) * dphi;
     }
-    for (int f = 1; f <= Nu; ++f) col(6)[f] = 1.0 / (Rf[f] - Rf[f - 1]);
-    for (int f = 0; f < Nu; ++f) col(7)[f] = 1.0 / (Rf[f + 1] - Rf[f]);
+    for (int f = 0; f <= Nu; ++f) {
+      double *c = t.data() + (size_t)kRow64W * f;
+      c[hAf] = Rf[f] * dphi;
+      if (f >= 1) c[hCl] = 0.5 / (Rf[f] - Rf[f - 1]);
+      if (f < Nu) c[hCr] = 0.5 / (Rf[f + 1] - Rf[f]);
+    }
     MK(dmalloc(&rowtab, t.size()));
     MK(cudaMemcpy(rowtab, t.data(), t.size() * sizeof(double), cudaMemcpyHostToDevice));
-    auto dc = [&](int k) { return (const double *)(rowtab + (size_t)k * (Nu + 1)); };
-    geom.gstar = dc(0); geom.invR = dc(1); geom.invdRc = dc(2); geom.invVol = dc(3);
-    geom.invdR = dc(4); geom.invdl = dc(5); geom.invdRl = dc(6); geom.invdRr = dc(7);
+    geom.rowtab = rowtab;
+    geom.invdR = rowtab + (size_t)kRow64W * (Nu + 1);
+    geom.invdl = geom.invdR + Nu;
   }
   geom.R = dR; geom.Rf = dRf; geom.Vol = dVol;
   geom.Nu = Nu; geom.Nphi = Nphi; geom.dphi = dphi; geom.du = du;
   geom.Kpoly = p.Kpoly; geom.gamma = p.gamma_gas; geom.gmstar = p.gmstar;
-  geom.inv2dphi = 1.0 / (2.0 * dphi); geom.invdu = 1.0 / du; geom.inv2du = 1.0 / (2.0 * du);
   geom.gamma2 = (p.gamma_gas == 2.0) ? 1 : 0;
   MK(prepare_fft_kernels());
   int rc = build_khat();

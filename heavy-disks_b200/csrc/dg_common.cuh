@@ -113,7 +113,8 @@ __device__ __forceinline__ T warp_sum(T v) {
   return v;
 }
 
-// Block-wide max that keeps NaN (fmax drops NaN, so NaN is tracked separately).
+// Block-wide max that keeps NaN (fmax drops NaN, so NaN is tracked separately).  NT: threads
+// of the block, 0 = blockDim.x.
 template <int NT>
 __device__ __forceinline__ double block_max_nan(double v, double *red) {
   bool bad = !(v == v);
@@ -126,7 +127,8 @@ __device__ __forceinline__ double block_max_nan(double v, double *red) {
   double r = 0.0;
   if (threadIdx.x == 0) {
     r = red[0];
-    for (int k = 1; k < NT / 32; ++k) {
+    const int nw = NT ? NT / 32 : (int)(blockDim.x >> 5);
+    for (int k = 1; k < nw; ++k) {
       double x = red[k];
       if (!(x == x) || !(r == r)) r = __longlong_as_double(0x7ff8000000000000ll);
       else r = fmax(r, x);

@@ -22,221 +22,187 @@ __device__ __forceinline__ void add_modes(double *msum, int nmodes, double s, in
 }
 
 // ---------------------------------------------------------------------------------
-__global__ void __launch_bounds__(kHydroThreads) k_hydro64(
-    const double *__restrict__ Sig, const double *__restrict__ vR, const double *__restrict__ vp,
-    const double *__restrict__ Phi, const double *__restrict__ gRin, const double *__restrict__ gpin, int force_mode,
-    double *__restrict__ So, double *__restrict__ vRo, double *__restrict__ vpo, Ctl *ctl, Geom64 g) {
-  __shared__ double sS[kLI][kLJ], sVR[kLI][kLJ], sVP[kLI][kLJ], sP[kLI][kLJ], sPh[kLI][kLJ];
-  __shared__ double sVR1[kSI][kSJ], sVP1[kSI][kSJ];
-  __shared__ double fF[kTI + 1][kSJ], fFR[kTI + 1][kSJ], fFP[kTI + 1][kSJ];
-  __shared__ double pF[3 * kTI][kTJ + 1];  // phi-face fluxes: rows [0,TI) F, [TI,2TI) FR, [2TI,3TI) FP
-  __shared__ double red[kHydroThreads / 32];
-  // transportR outputs reuse the (dead after the source stage) pressure / velocity tiles
-  double(*s2S)[kLJ] = sP;
-  double(*s2VR)[kLJ] = sVR;
-  double(*s2VP)[kLJ] = sVP;
+__device__ __forceinline__ double up1(double v) { return __shfl_up_sync(0xffffffffu, v, 1); }
+__device__ __forceinline__ double dn1(double v) { return __shfl_down_sync(0xffffffffu, v, 1); }
 
-  const int Nu = g.Nu, Nphi = g.Nphi;
-  const int i0 = blockIdx.y * kTI, j0 = blockIdx.x * kTJ;
+// One time step (hydro64.cuh).  blockIdx.x: group of blockDim.x / 32 strips; blockIdx.y: band
+// of `band` rows.
+template <bool G2, int FM>
+__global__ void __launch_bounds__(32 * kMaxWarps64, 3) k_hydro64(
+    const double *__restrict__ Sig, const double *__restrict__ vR, const double *__restrict__ vp,
+    const double *__restrict__ Phi, const double *__restrict__ gRin, const double *__restrict__ gpin,
+    double *__restrict__ So, double *__restrict__ vRo, double *__restrict__ vpo, Ctl *ctl, const Geom64 g, int band) {
+  __shared__ __align__(16) double tab[(kMaxBand64 + 6) * kRow64W];
+  __shared__ double red[kMaxWarps64];
+  const int Nu = g.Nu, Nphi = g.Nphi, tid = threadIdx.x, lane = tid & 31, nt = blockDim.x;
+  const int iA = blockIdx.y * band, iB = min(iA + band, Nu);
+  const int strip = blockIdx.x * (nt >> 5) + (tid >> 5), j0 = strip * kOutCols64;
+  int j = (j0 - kHalo64 + lane) % Nphi;
+  if (j < 0) j += Nphi;
+  const bool live = j0 < Nphi;
+  const bool outp = live && lane >= kHalo64 && lane < kHalo64 + kOutCols64 && j0 - kHalo64 + lane < Nphi;
+
+  pdl_wait();  // dt, the state and the potential come from earlier kernels on the stream
+  pdl_trigger();
   const StepInfo si = read_step_info(ctl, true);
   const double dt = si.dt;
-  const int tid = threadIdx.x;
-  double msum[2 * kMaxModes];
-#pragma unroll
-  for (int q = 0; q < 2 * kMaxModes; ++q) msum[q] = 0.0;
+  double msum[2 * kMaxModes];  // set only when the launch accumulates modes
   double lmax = 0.0;
+  bool bad = false;
 
   if (!si.active) {
     // pass-through so a launch after the loop has ended leaves the state unchanged
-    for (int c = tid; c < kTI * kTJ; c += kHydroThreads) {
-      int i = i0 + c / kTJ, j = j0 + c % kTJ;
-      if (i < Nu && j < Nphi) {
-        size_t k = (size_t)i * Nphi + j;
+    if (outp)
+      for (int i = iA; i < iB; ++i) {
+        const size_t k = (size_t)i * Nphi + j;
         So[k] = Sig[k]; vRo[k] = vR[k]; vpo[k] = vp[k];
         lmax = fmax(lmax, cfl_rate64(g, i, So[k], vRo[k], vpo[k]));
       }
-    }
-    finish_launch<kHydroThreads>(ctl, si, lmax, msum, red);
+    finish_launch<0>(ctl, si, lmax, msum, red);
     return;
   }
 
-  // ---- load the halo region ----
-  for (int c = tid; c < kLI * kLJ; c += kHydroThreads) {
-    int li = c / kLJ, lj = c % kLJ;
-    int i = i0 - kH + li;
-    int j = j0 - kH + lj;
-    j = ((j % Nphi) + Nphi) % Nphi;
-    double s = 0.0, a = 0.0, b = 0.0, ph = 0.0;
-    if (i >= 0 && i < Nu) {
-      size_t k = (size_t)i * Nphi + j;
-      s = Sig[k]; a = vR[k]; b = vp[k];
-      if (force_mode == kForcePhi) ph = Phi[k];
-    }
-    sS[li][lj] = s; sVR[li][lj] = a; sVP[li][lj] = b; sPh[li][lj] = ph;
-    sP[li][lj] = (i >= 0 && i < Nu) ? pres64(g, s) : 0.0;
+  // row constants of rows iA-3 .. iB+2 (edge rows repeat), products with dt included
+  for (int c = tid; c < (iB - iA + 6) * kRow64W; c += nt) {
+    const int q = c % kRow64W, i = iA - 3 + c / kRow64W;
+    // faces f = 0 .. Nu; row constants of the rows outside the grid are the edge rows'
+    const bool face = q == hAf || q == hCl || q == hCr;
+    const int row = max(0, min(i, face ? Nu : Nu - 1));
+    const double v = g.rowtab[(size_t)row * kRow64W + q];
+    tab[c] = (q == hCvol || q == hCphi || q == hCl || q == hCr) ? dt * v : v;
   }
   __syncthreads();
 
-  // ---- source (hydro.hpp:73-96) on rows i0-2 .. i0+TI+1 ----
-  for (int c = tid; c < kSI * kSJ; c += kHydroThreads) {
-    int si_ = c / kSJ, sj = c % kSJ;
-    int i = i0 - 2 + si_;
-    int li = si_ + 1, lj = sj + 1;
-    double nvr = 0.0, nvp = 0.0;
-    if (i >= 0 && i < Nu) {
-      int im = i - 1 > 0 ? i - 1 : 0, ip = i + 1 < Nu - 1 ? i + 1 : Nu - 1;
-      int lim = li + (im - i), lip = li + (ip - i);
-      double Ri = g.R[i], iR = g.invR[i];
-      double s = sS[li][lj];
-      double dPdR = (sP[lip][lj] - sP[lim][lj]) * g.invdRc[i];
-      double dPdphi = (sP[li][lj + 1] - sP[li][lj - 1]) * g.inv2dphi;
-      double gR = g.gstar[i];
-      double gp = 0.0;
-      if (force_mode == kForcePhi) {  // kalnajs.hpp:71-78
-        double dPhidphi = (sPh[li][lj + 1] - sPh[li][lj - 1]) * g.inv2dphi;
-        double dPhidu;
-        if (i == 0) dPhidu = (sPh[li + 1][lj] - sPh[li][lj]) * g.invdu;
-        else if (i == Nu - 1) dPhidu = (sPh[li][lj] - sPh[li - 1][lj]) * g.invdu;
-        else dPhidu = (sPh[li + 1][lj] - sPh[li - 1][lj]) * g.inv2du;
-        gR += -dPhidu * iR;
-        gp += -dPhidphi * iR;
-      } else if (force_mode == kForceArrays) {
-        int j = ((j0 - 2 + sj) % Nphi + Nphi) % Nphi;
-        size_t k = (size_t)i * Nphi + j;
-        gR += gRin[k];
-        gp += gpin[k];
+  if (live) {
+    auto at = [&](int r) { return max(0, min(r, Nu - 1)) * Nphi + j; };  // at most 4096 x 8192
+    auto pres = [&](double s) { return G2 ? g.Kpoly * (s * s) : g.Kpoly * pow(s, g.gamma); };
+    const double cs2c = g.gamma * g.Kpoly;
+    int r = iA - 3;
+    // the next row, in flight
+    int x = at(r);
+    double nS = Sig[x], nU = vR[x], nW = vp[x], nPh = FM == kForcePhi ? Phi[x] : 0.0;
+    // row r-1 as loaded; pressure and potential of rows r-1 and r-2
+    double S1 = 0, U1 = 0, W1 = 0, P1 = 0, P2 = 0, Ph1 = 0, Ph2 = 0;
+    // rows r-2 and r-3 after the source; differences (row r-2) - (row r-3); slopes of row r-3
+    double S2 = 0, u2 = 0, w2 = 0, S3 = 0, u3 = 0, w3 = 0, dS = 0, du = 0, dw = 0, kS = 0, kU = 0, kW = 0;
+    // fluxes through the face between rows r-4 and r-3
+    double F0 = 0, FR0 = 0, FP0 = 0, tsum = 0;
+    const double *tc = tab;  // constants of row r
+#pragma unroll 2  // the windows' shifts become renames
+    for (int k = 0; r <= iB + 2; ++k, ++r, tc += kRow64W) {
+      const double S = nS, U = nU, W = nW, Ph = nPh;
+      x = at(r + 1);
+      nS = Sig[x]; nU = vR[x]; nW = vp[x];
+      if (FM == kForcePhi) nPh = Phi[x];
+      const double P = pres(S);
+      double s1 = 0, u1 = 0, w1 = 0;  // row r-1 after the source
+      if (k >= 2) {
+        // ---- source of row r-1 (hydro.hpp:73-96; kalnajs.hpp:71-78 for the forces) ----
+        const double *t = tc - kRow64W;
+        const double dPR = P - P2, dPp = dn1(P1) - up1(P1);
+        double aR = t[hGstar], gp = 0.0;
+        if (FM == kForcePhi) {
+          aR = fma(Ph - Ph2, t[hPhiu], aR);
+          gp = dn1(Ph1) - up1(Ph1);  // times -1 / (2 R dphi) below
+        } else if (FM == kForceArrays) {
+          aR += gRin[at(r - 1)];
+        }
+        double rs, tR = dPR * t[hInvdRc];
+        if (rcp_ok64(S1)) rs = rcp64(S1);
+        else rs = 1.0 / S1;
+        aR = fma(-tR, rs, aR);
+        const double wR = W1 * t[hInvR];
+        aR = fma(W1, wR, aR);
+        double ap = fma(t[hPhip], fma(dPp, rs, gp), -(U1 * wR));
+        if (FM == kForceArrays) ap += gpin[at(r - 1)];
+        s1 = S1;
+        u1 = fma(dt, aR, U1);
+        w1 = fma(dt, ap, W1);
       }
-      double vrc = sVR[li][lj], vpc = sVP[li][lj];
-      double aR = -dPdR / s + gR + vpc * vpc * iR;
-      double ap = -(1.0 / (s * Ri)) * dPdphi + gp - vrc * vpc * iR;
-      nvr = vrc + dt * aR;
-      nvp = vpc + dt * ap;
-    }
-    sVR1[si_][sj] = nvr;
-    sVP1[si_][sj] = nvp;
-  }
-  __syncthreads();
-
-  // ---- transportR fluxes (hydro.hpp:107-130) at faces f = i0 .. i0+TI ----
-  // cell index i in source coordinates: si_ = i - (i0 - 2); Sigma at sS[si_ + 1][sj + 1]
-  auto Ssrc = [&](int i, int sj) { return sS[i - (i0 - 2) + 1][sj + 1]; };
-  auto VRsrc = [&](int i, int sj) { return sVR1[i - (i0 - 2)][sj]; };
-  auto VPsrc = [&](int i, int sj) { return sVP1[i - (i0 - 2)][sj]; };
-  for (int c = tid; c < (kTI + 1) * kSJ; c += kHydroThreads) {
-    int fi = c / kSJ, sj = c % kSJ;
-    int f = i0 + fi;
-    double F = 0.0, FR = 0.0, FP = 0.0;
-    if (f >= 1 && f <= Nu - 1) {
-      double Af = g.Rf[f] * g.dphi;
-      double idRl = g.invdRl[f], idRr = g.invdRr[f];
-      double vf = 0.5 * (VRsrc(f - 1, sj) + VRsrc(f, sj));
-      double sf, vRf, vpf;
-      if (vf > 0) {
-        int u = f - 1;
-        bool sl = (u > 0 && u < Nu - 1);
-        double kS = sl ? vanleer64(Ssrc(u + 1, sj) - Ssrc(u, sj), Ssrc(u, sj) - Ssrc(u - 1, sj)) : 0.0;
-        double kR = sl ? vanleer64(VRsrc(u + 1, sj) - VRsrc(u, sj), VRsrc(u, sj) - VRsrc(u - 1, sj)) : 0.0;
-        double kP = sl ? vanleer64(VPsrc(u + 1, sj) - VPsrc(u, sj), VPsrc(u, sj) - VPsrc(u - 1, sj)) : 0.0;
-        sf = Ssrc(u, sj) + 0.5 * kS * (1.0 - vf * dt * idRl);
-        vRf = VRsrc(u, sj) + 0.5 * kR * (1.0 - vf * dt * idRl);
-        vpf = VPsrc(u, sj) + 0.5 * kP * (1.0 - vf * dt * idRl);
-      } else {
-        int u = f;
-        bool sl = (u > 0 && u < Nu - 1);
-        double kS = sl ? vanleer64(Ssrc(u + 1, sj) - Ssrc(u, sj), Ssrc(u, sj) - Ssrc(u - 1, sj)) : 0.0;
-        double kR = sl ? vanleer64(VRsrc(u + 1, sj) - VRsrc(u, sj), VRsrc(u, sj) - VRsrc(u - 1, sj)) : 0.0;
-        double kP = sl ? vanleer64(VPsrc(u + 1, sj) - VPsrc(u, sj), VPsrc(u, sj) - VPsrc(u - 1, sj)) : 0.0;
-        sf = Ssrc(u, sj) - 0.5 * kS * (1.0 + vf * dt * idRr);
-        vRf = VRsrc(u, sj) - 0.5 * kR * (1.0 + vf * dt * idRr);
-        vpf = VPsrc(u, sj) - 0.5 * kP * (1.0 + vf * dt * idRr);
+      const double eS = s1 - S2, eU = u1 - u2, eW = w1 - w2;  // (row r-1) - (row r-2)
+      double lS = 0, lU = 0, lW = 0;                          // slopes of row r-2
+      double F = 0, FR = 0, FP = 0;                           // face between rows r-3 and r-2
+      if (k >= 4) {
+        if (r - 2 > 0 && r - 2 < Nu - 1) {  // no slope in the first and last row (hydro.hpp:117-119)
+          lS = vanleer64(eS, dS);
+          lU = vanleer64(eU, du);
+          lW = vanleer64(eW, dw);
+        }
+        // ---- radial flux (hydro.hpp:107-130) through face f = r-2 ----
+        if (k >= 5 && r - 2 >= 1 && r - 2 <= Nu - 1) {
+          const double *t = tc - 2 * kRow64W;
+          const double vf = 0.5 * (u3 + u2);
+          const bool up = pos64(vf);
+          // q_u + k_u (+-1/2 - vf dt / (2 dR_u))
+          const double h = fma(-vf, up ? t[hCl] : t[hCr], up ? 0.5 : -0.5);
+          const double sf = fma(h, up ? kS : lS, up ? S3 : S2);
+          const double uf = fma(h, up ? kU : lU, up ? u3 : u2);
+          const double wf = fma(h, up ? kW : lW, up ? w3 : w2);
+          F = vf * sf * t[hAf];
+          FR = F * uf;
+          FP = F * wf;
+        }
+        if (k >= 6) {
+          // ---- row i = r-3: radial gather (hydro.hpp:131-139) ----
+          const double *t = tc - 3 * kRow64W;
+          const double cv = t[hCvol];
+          const double ns = fma(cv, F0 - F, S3);
+          const double mR = fma(cv, FR0 - FR, S3 * u3), mP = fma(cv, FP0 - FP, S3 * w3);
+          double d = dmax_ref(ns, 1e-10);
+          double y = rcp_approx64(d);
+          const double a = quot64(mR, d, y), b = quot64(mP, d, y);
+          // ---- azimuthal sweep (hydro.hpp:150-178): this lane's left face and cell ----
+          const double sm = up1(ns), am = up1(a), bm = up1(b);
+          const double qS = vanleer64(dn1(ns) - ns, ns - sm), qA = vanleer64(dn1(a) - a, a - am),
+                       qB = vanleer64(dn1(b) - b, b - bm);
+          const double qSm = up1(qS), qAm = up1(qA), qBm = up1(qB);
+          const double vf = 0.5 * (bm + b);
+          const bool up = pos64(vf);
+          const double h = fma(-vf, t[hCphi], up ? 0.5 : -0.5);
+          const double sf = fma(h, up ? qSm : qS, up ? sm : ns);
+          const double af = fma(h, up ? qAm : qA, up ? am : a);
+          const double bf = fma(h, up ? qBm : qB, up ? bm : b);
+          const double G = vf * sf * t[hAphi], GR = G * af, GP = G * bf;
+          const double n2 = fma(cv, G - dn1(G), ns);
+          const double mR2 = fma(cv, GR - dn1(GR), ns * a), mP2 = fma(cv, GP - dn1(GP), ns * b);
+          d = dmax_ref(n2, 1e-10);  // the quotients' floor and the state's (hydro.hpp:69)
+          y = rcp_approx64(d);
+          const double uo = quot64(mR2, d, y), wo = quot64(mP2, d, y);
+          if (outp) {
+            const int q = (r - 3) * Nphi + j;
+            So[q] = d;
+            vRo[q] = uo;
+            vpo[q] = wo;
+            // CFL rate of the new state (hydro.hpp:54-57); d is above the 1e-12 of cs
+            const double cs = sqrt(G2 ? cs2c * d : cs2c * pow(d, g.gamma - 1.0));
+            const double rate = fma(fabs(uo) + cs, t[hInvdR], (fabs(wo) + cs) * t[hInvdl]);
+            bad |= !(rate == rate) || !(uo == uo) || !(wo == wo);
+            lmax = fmax(lmax, rate);
+            if (si.nmodes) tsum = fma(d, t[hDA], tsum);
+          }
+        }
       }
-      double fm = vf * sf * Af;
-      F = fm; FR = fm * vRf; FP = fm * vpf;
+      F0 = F; FR0 = FR; FP0 = FP;
+      S3 = S2; u3 = u2; w3 = w2; kS = lS; kU = lU; kW = lW;
+      S2 = s1; u2 = u1; w2 = w1; dS = eS; du = eU; dw = eW;
+      S1 = S; U1 = U; W1 = W;
+      P2 = P1; P1 = P; Ph2 = Ph1; Ph1 = Ph;
     }
-    fF[fi][sj] = F; fFR[fi][sj] = FR; fFP[fi][sj] = FP;
-  }
-  __syncthreads();
-
-  // ---- transportR gather (hydro.hpp:131-139) on rows i0 .. i0+TI-1 ----
-  for (int c = tid; c < kTI * kSJ; c += kHydroThreads) {
-    int ri = c / kSJ, sj = c % kSJ;
-    int i = i0 + ri;
-    double ns = 0.0, a = 0.0, b = 0.0;
-    if (i < Nu) {
-      double s = Ssrc(i, sj), vr1 = VRsrc(i, sj), vp1 = VPsrc(i, sj);
-      double mR = s * vr1, mp = s * vp1;
-      double iV = g.invVol[i];
-      ns = s + dt * (fF[ri][sj] - fF[ri + 1][sj]) * iV;
-      double nmR = mR + dt * (fFR[ri][sj] - fFR[ri + 1][sj]) * iV;
-      double nmP = mp + dt * (fFP[ri][sj] - fFP[ri + 1][sj]) * iV;
-      double d = dmax_ref(ns, 1e-10);
-      a = nmR / d;
-      b = nmP / d;
-    }
-    s2S[ri][sj] = ns; s2VR[ri][sj] = a; s2VP[ri][sj] = b;
-  }
-  __syncthreads();
-
-  // ---- transportPhi fluxes (hydro.hpp:150-169): face pj is j-1/2 of cell j0+pj ----
-  // cells in R-output coordinates: column c <-> global j0 - 2 + c
-  for (int c = tid; c < kTI * (kTJ + 1); c += kHydroThreads) {
-    int ri = c / (kTJ + 1), pj = c % (kTJ + 1);
-    int i = i0 + ri;
-    double F = 0.0, FR = 0.0, FP = 0.0;
-    if (i < Nu) {
-      double idl = g.invdl[i], Aface = g.Rf[i + 1] - g.Rf[i];
-      int cm = pj + 1, cc = pj + 2;  // cells j-1, j
-      double vf = 0.5 * (s2VP[ri][cm] + s2VP[ri][cc]);
-      double sf, vRf, vpf;
-      int u = (vf > 0) ? cm : cc;
-      double kS = vanleer64(s2S[ri][u + 1] - s2S[ri][u], s2S[ri][u] - s2S[ri][u - 1]);
-      double kR = vanleer64(s2VR[ri][u + 1] - s2VR[ri][u], s2VR[ri][u] - s2VR[ri][u - 1]);
-      double kP = vanleer64(s2VP[ri][u + 1] - s2VP[ri][u], s2VP[ri][u] - s2VP[ri][u - 1]);
-      if (vf > 0) {
-        sf = s2S[ri][u] + 0.5 * kS * (1.0 - vf * dt * idl);
-        vRf = s2VR[ri][u] + 0.5 * kR * (1.0 - vf * dt * idl);
-        vpf = s2VP[ri][u] + 0.5 * kP * (1.0 - vf * dt * idl);
-      } else {
-        sf = s2S[ri][u] - 0.5 * kS * (1.0 + vf * dt * idl);
-        vRf = s2VR[ri][u] - 0.5 * kR * (1.0 + vf * dt * idl);
-        vpf = s2VP[ri][u] - 0.5 * kP * (1.0 + vf * dt * idl);
-      }
-      double fm = vf * sf * Aface;
-      F = fm; FR = fm * vRf; FP = fm * vpf;
-    }
-    pF[ri][pj] = F; pF[kTI + ri][pj] = FR; pF[2 * kTI + ri][pj] = FP;
-  }
-  __syncthreads();
-
-  // ---- transportPhi gather (hydro.hpp:170-178) + floor (:69) + next-step CFL ----
-  bool bad = false;
-  for (int c = tid; c < kTI * kTJ; c += kHydroThreads) {
-    int ri = c / kTJ, pj = c % kTJ;
-    int i = i0 + ri, j = j0 + pj;
-    if (i < Nu && j < Nphi) {
-      int cc = pj + 2;
-      double s = s2S[ri][cc], vr = s2VR[ri][cc], vpp = s2VP[ri][cc];
-      double mR = s * vr, mp = s * vpp;
-      double iV = g.invVol[i];
-      double ns = s + dt * (pF[ri][pj] - pF[ri][pj + 1]) * iV;
-      double nmR = mR + dt * (pF[kTI + ri][pj] - pF[kTI + ri][pj + 1]) * iV;
-      double nmP = mp + dt * (pF[2 * kTI + ri][pj] - pF[2 * kTI + ri][pj + 1]) * iV;
-      double d = dmax_ref(ns, 1e-10);
-      double vro = nmR / d, vpo_ = nmP / d;
-      double so = dmax_ref(ns, 1e-10);
-      size_t k = (size_t)i * Nphi + j;
-      So[k] = so; vRo[k] = vro; vpo[k] = vpo_;
-      double rate = cfl_rate64(g, i, so, vro, vpo_);
-      bad |= !(rate == rate) || !(vro == vro) || !(vpo_ == vpo_);
-      lmax = fmax(lmax, rate);
-      if (si.nmodes) {
-        double dA = g.R[i] * (g.Rf[i + 1] - g.Rf[i]) * g.dphi;
-        add_modes(msum, si.nmodes, so, j, g.dphi, dA);
+    // mode sums of the column (diskmain.cpp:76-80): Sigma dA summed over the band's rows
+    if (si.nmodes) {
+      const double phi = (j + 0.5) * g.dphi;
+      for (int m = 0; m < si.nmodes; ++m) {
+        double sn, cs;
+        sincos(m * phi, &sn, &cs);
+        msum[2 * m] = tsum * cs;
+        msum[2 * m + 1] = -tsum * sn;
       }
     }
+  } else {
+    for (int q = 0; q < 2 * si.nmodes; ++q) msum[q] = 0.0;
   }
   if (bad) lmax = __longlong_as_double(0x7ff8000000000000ll);
-  finish_launch<kHydroThreads>(ctl, si, lmax, msum, red);
+  finish_launch<0>(ctl, si, lmax, msum, red);
 }
 
 // CFL reduction over a state (DiskHydro::timestep, hydro.hpp:48-61); the last CTA stores
@@ -365,9 +331,29 @@ static int sm_count() {
 cudaError_t launch_hydro64(const double *Sig, const double *vR, const double *vp, const double *Phi,
                            const double *gR, const double *gp, int force_mode, double *So, double *vRo, double *vpo,
                            Ctl *ctl, const Geom64 &g, cudaStream_t st) {
-  dim3 grid((g.Nphi + kTJ - 1) / kTJ, (g.Nu + kTI - 1) / kTI);
-  k_hydro64<<<grid, kHydroThreads, 0, st>>>(Sig, vR, vp, Phi, gR, gp, force_mode, So, vRo, vpo, ctl, g);
-  return cudaGetLastError();
+  // strips per CTA: the count that leaves the fewest idle warps; rows per band: the GPU's
+  // warps (16 per SM) shared among the strips.  A grid too small to fill the GPU takes
+  // one-row bands: seven row visits for one, but the shortest chain (128^2 step: 19.99 us,
+  // 21.15 with at least two rows, 23.21 with four).
+  const int strips = (g.Nphi + kOutCols64 - 1) / kOutCols64;
+  int wc = strips <= kMaxWarps64 ? strips : 4;
+  if (strips > kMaxWarps64)
+    for (int c : {5, 3})
+      if ((strips + c - 1) / c * c < (strips + wc - 1) / wc * wc) wc = c;
+  const int cols = (strips + wc - 1) / wc, slots = sm_count() * (16 / wc);  // 16 warps per SM
+  int bands = slots / cols;
+  if (bands < 1) bands = 1;
+  int band = (g.Nu + bands - 1) / bands;
+  if (band < 1) band = 1;
+  if (band > kMaxBand64) band = kMaxBand64;
+  auto go = [&](auto kern) {
+    return launch_pdl(kern, dim3(cols, (g.Nu + band - 1) / band), dim3(32 * wc), 0, st, Sig, vR, vp, Phi, gR, gp, So,
+                      vRo, vpo, ctl, g, band);
+  };
+  if (force_mode == kForcePhi) return g.gamma2 ? go(k_hydro64<true, kForcePhi>) : go(k_hydro64<false, kForcePhi>);
+  if (force_mode == kForceArrays)
+    return g.gamma2 ? go(k_hydro64<true, kForceArrays>) : go(k_hydro64<false, kForceArrays>);
+  return g.gamma2 ? go(k_hydro64<true, kForceNone>) : go(k_hydro64<false, kForceNone>);
 }
 
 cudaError_t launch_cfl64(const double *Sig, const double *vR, const double *vp, Ctl *ctl, const Geom64 &g,

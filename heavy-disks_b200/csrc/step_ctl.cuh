@@ -64,7 +64,8 @@ __device__ __forceinline__ StepInfo read_step_info(const Ctl *ctl, bool advance_
 }
 
 // A CTA's share of the launch: its CFL max and mode sums, folded into the control block
-// with fire-and-forget atomics (the result of thread 0's block reduction).
+// with fire-and-forget atomics (the result of thread 0's block reduction).  NT as in
+// block_max_nan; msum is read only when the launch accumulates modes.
 template <int NT>
 __device__ __forceinline__ double fold_launch_sums(Ctl *ctl, const StepInfo &si, double local_max, const double *msum,
                                                    double *red) {
@@ -76,7 +77,8 @@ __device__ __forceinline__ double fold_launch_sums(Ctl *ctl, const StepInfo &si,
     __syncthreads();
     if (threadIdx.x == 0) {
       double s = 0.0;
-      for (int k = 0; k < NT / 32; ++k) s += red[k];
+      const int nw = NT ? NT / 32 : (int)(blockDim.x >> 5);
+      for (int k = 0; k < nw; ++k) s += red[k];
       atomicAdd(&ctl->modesum[q], s);
     }
     __syncthreads();
