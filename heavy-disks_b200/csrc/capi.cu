@@ -112,6 +112,8 @@ int dg_handle::init(const dg_params &pp) {
     MK(cudaMemset(VR[b], 0, n * sizeof(double)));
     MK(cudaMemset(VP[b], 0, n * sizeof(double)));
   }
+  if (p.precision == DG_PREC_FP64 && p.gamma_gas != 2.0)
+    for (int b = 0; b < 2; ++b) MK(dmalloc(&PR[b], n));
   MK(dmalloc(&dPhi, n)); MK(dmalloc(&gA, n)); MK(dmalloc(&gB, n));
   ldW = Nu + (Nu & 1);
   MK(dmalloc(&W, (size_t)Nc * ldW)); MK(dmalloc(&Khat, (size_t)Nc * M));
@@ -209,7 +211,7 @@ void dg_handle::release() {
   mixed_release();
   if (graph_exec) cudaGraphExecDestroy(graph_exec);
   if (diag) cudaFree(diag);
-  void *ptrs[] = {rowtab, dR, dRf, dVol, dSqrtR, dR32, S[0], S[1], VR[0], VR[1], VP[0], VP[1], dPhi, gA, gB,
+  void *ptrs[] = {rowtab, dR, dRf, dVol, dSqrtR, dR32, S[0], S[1], VR[0], VR[1], VP[0], VP[1], PR[0], PR[1], dPhi, gA, gB,
                   W, Khat, twPhi, scratch, ctl};
   for (void *q : ptrs)
     if (q) cudaFree(q);
@@ -249,7 +251,8 @@ int dg_handle::enqueue_step() {
     fm = kForcePhi;
   }
   MK(prof_begin(DG_PROF_HYDRO));
-  MK(launch_hydro64(S[c], VR[c], VP[c], dPhi, nullptr, nullptr, fm, S[o], VR[o], VP[o], ctl, geom, st));
+  MK(launch_hydro64(S[c], VR[c], VP[c], dPhi, nullptr, nullptr, fm, PR[c], S[o], VR[o], VP[o], PR[o], ctl, geom,
+                    st));
   MK(prof_end(DG_PROF_HYDRO));
   cur = o;
   return DG_OK;
@@ -359,7 +362,7 @@ int dg_handle::enqueue_step_forces(const double *gRh, const double *gph) {
     fm = kForceArrays;
   }
   const int c = cur, o = cur ^ 1;
-  MK(launch_hydro64(S[c], VR[c], VP[c], nullptr, gA, gB, fm, S[o], VR[o], VP[o], ctl, geom, st));
+  MK(launch_hydro64(S[c], VR[c], VP[c], nullptr, gA, gB, fm, PR[c], S[o], VR[o], VP[o], PR[o], ctl, geom, st));
   cur = o;
   return DG_OK;
 }
@@ -382,6 +385,7 @@ int dg_handle::upload_state(const double *Sig, const double *vRh, const double *
   MK(cudaMemcpyAsync(S[cur], Sig, n * sizeof(double), cudaMemcpyHostToDevice, st));
   MK(cudaMemcpyAsync(VR[cur], vRh, n * sizeof(double), cudaMemcpyHostToDevice, st));
   MK(cudaMemcpyAsync(VP[cur], vph, n * sizeof(double), cudaMemcpyHostToDevice, st));
+  if (PR[cur]) MK(launch_pressure64(S[cur], PR[cur], geom, st));
   return DG_OK;
 }
 

@@ -38,6 +38,7 @@ struct dg_handle {
 
   // plain-method state (ping-pong), forces scratch, gravity workspace
   double *S[2] = {nullptr, nullptr}, *VR[2] = {nullptr, nullptr}, *VP[2] = {nullptr, nullptr};
+  double *PR[2] = {nullptr, nullptr};  // pressure of S[.] (FP64 path, Gamma != 2)
   int cur = 0;
   double *dPhi = nullptr, *gA = nullptr, *gB = nullptr;
   // phi half spectra [m][i], row stride ldW (Nu rounded up to even); the real khat table

@@ -31,7 +31,8 @@ template <bool G2, int FM>
 __global__ void __launch_bounds__(32 * kMaxWarps64, 3) k_hydro64(
     const double *__restrict__ Sig, const double *__restrict__ vR, const double *__restrict__ vp,
     const double *__restrict__ Phi, const double *__restrict__ gRin, const double *__restrict__ gpin,
-    double *__restrict__ So, double *__restrict__ vRo, double *__restrict__ vpo, Ctl *ctl, const Geom64 g, int band) {
+    const double *__restrict__ Pin, double *__restrict__ So, double *__restrict__ vRo, double *__restrict__ vpo,
+    double *__restrict__ Po, Ctl *ctl, const Geom64 g, int band) {
   __shared__ __align__(16) double tab[(kMaxBand64 + 6) * kRow64W];
   __shared__ double red[kMaxWarps64];
   const int Nu = g.Nu, Nphi = g.Nphi, tid = threadIdx.x, lane = tid & 31, nt = blockDim.x;
@@ -56,6 +57,7 @@ __global__ void __launch_bounds__(32 * kMaxWarps64, 3) k_hydro64(
       for (int i = iA; i < iB; ++i) {
         const size_t k = (size_t)i * Nphi + j;
         So[k] = Sig[k]; vRo[k] = vR[k]; vpo[k] = vp[k];
+        if (!G2) Po[k] = Pin[k];
         lmax = fmax(lmax, cfl_rate64(g, i, So[k], vRo[k], vpo[k]));
       }
     finish_launch<0>(ctl, si, lmax, msum, red);
@@ -75,12 +77,10 @@ __global__ void __launch_bounds__(32 * kMaxWarps64, 3) k_hydro64(
 
   if (live) {
     auto at = [&](int r) { return max(0, min(r, Nu - 1)) * Nphi + j; };  // at most 4096 x 8192
-    auto pres = [&](double s) { return G2 ? g.Kpoly * (s * s) : g.Kpoly * pow(s, g.gamma); };
-    const double cs2c = g.gamma * g.Kpoly;
     int r = iA - 3;
     // the next row, in flight
     int x = at(r);
-    double nS = Sig[x], nU = vR[x], nW = vp[x], nPh = FM == kForcePhi ? Phi[x] : 0.0;
+    double nS = Sig[x], nU = vR[x], nW = vp[x], nP = G2 ? 0.0 : Pin[x], nPh = FM == kForcePhi ? Phi[x] : 0.0;
     // row r-1 as loaded; pressure and potential of rows r-1 and r-2
     double S1 = 0, U1 = 0, W1 = 0, P1 = 0, P2 = 0, Ph1 = 0, Ph2 = 0;
     // rows r-2 and r-3 after the source; differences (row r-2) - (row r-3); slopes of row r-3
@@ -90,11 +90,11 @@ __global__ void __launch_bounds__(32 * kMaxWarps64, 3) k_hydro64(
     const double *tc = tab;  // constants of row r
 #pragma unroll 2  // the windows' shifts become renames
     for (int k = 0; r <= iB + 2; ++k, ++r, tc += kRow64W) {
-      const double S = nS, U = nU, W = nW, Ph = nPh;
+      const double S = nS, U = nU, W = nW, Ph = nPh, P = G2 ? g.Kpoly * (S * S) : nP;
       x = at(r + 1);
       nS = Sig[x]; nU = vR[x]; nW = vp[x];
+      if (!G2) nP = Pin[x];
       if (FM == kForcePhi) nPh = Phi[x];
-      const double P = pres(S);
       double s1 = 0, u1 = 0, w1 = 0;  // row r-1 after the source
       if (k >= 2) {
         // ---- source of row r-1 (hydro.hpp:73-96; kalnajs.hpp:71-78 for the forces) ----
@@ -173,9 +173,10 @@ __global__ void __launch_bounds__(32 * kMaxWarps64, 3) k_hydro64(
             So[q] = d;
             vRo[q] = uo;
             vpo[q] = wo;
-            // CFL rate of the new state (hydro.hpp:54-57); d is above the 1e-12 of cs
-            const double cs = sqrt(G2 ? cs2c * d : cs2c * pow(d, g.gamma - 1.0));
-            const double rate = fma(fabs(uo) + cs, t[hInvdR], (fabs(wo) + cs) * t[hInvdl]);
+            double Pn = 0.0;
+            if (!G2) Po[q] = Pn = pres64(g, d);
+            // CFL rate of the new state; d is above the 1e-12 of the reference's cs
+            const double rate = rate64(uo, wo, cs64(g, d, Pn), t[hInvdR], t[hInvdl]);
             bad |= !(rate == rate) || !(uo == uo) || !(wo == wo);
             lmax = fmax(lmax, rate);
             if (si.nmodes) tsum = fma(d, t[hDA], tsum);
@@ -329,8 +330,8 @@ static int sm_count() {
 }
 
 cudaError_t launch_hydro64(const double *Sig, const double *vR, const double *vp, const double *Phi,
-                           const double *gR, const double *gp, int force_mode, double *So, double *vRo, double *vpo,
-                           Ctl *ctl, const Geom64 &g, cudaStream_t st) {
+                           const double *gR, const double *gp, int force_mode, const double *Pin, double *So,
+                           double *vRo, double *vpo, double *Po, Ctl *ctl, const Geom64 &g, cudaStream_t st) {
   // strips per CTA: the count that leaves the fewest idle warps; rows per band: the GPU's
   // warps (16 per SM) shared among the strips.  A grid too small to fill the GPU takes
   // one-row bands: seven row visits for one, but the shortest chain (128^2 step: 19.99 us,
@@ -347,13 +348,28 @@ cudaError_t launch_hydro64(const double *Sig, const double *vR, const double *vp
   if (band < 1) band = 1;
   if (band > kMaxBand64) band = kMaxBand64;
   auto go = [&](auto kern) {
-    return launch_pdl(kern, dim3(cols, (g.Nu + band - 1) / band), dim3(32 * wc), 0, st, Sig, vR, vp, Phi, gR, gp, So,
-                      vRo, vpo, ctl, g, band);
+    return launch_pdl(kern, dim3(cols, (g.Nu + band - 1) / band), dim3(32 * wc), 0, st, Sig, vR, vp, Phi, gR, gp, Pin,
+                      So, vRo, vpo, Po, ctl, g, band);
   };
   if (force_mode == kForcePhi) return g.gamma2 ? go(k_hydro64<true, kForcePhi>) : go(k_hydro64<false, kForcePhi>);
   if (force_mode == kForceArrays)
     return g.gamma2 ? go(k_hydro64<true, kForceArrays>) : go(k_hydro64<false, kForceArrays>);
   return g.gamma2 ? go(k_hydro64<true, kForceNone>) : go(k_hydro64<false, kForceNone>);
+}
+
+// the pressure field of a state (Gamma != 2)
+__global__ void k_pressure64(const double *__restrict__ Sig, double *__restrict__ P, Geom64 g) {
+  const size_t n = (size_t)g.Nu * g.Nphi;
+  for (size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x)
+    P[k] = pres64(g, Sig[k]);
+}
+
+cudaError_t launch_pressure64(const double *Sig, double *P, const Geom64 &g, cudaStream_t st) {
+  const size_t n = (size_t)g.Nu * g.Nphi;
+  int blocks = (int)((n + 255) / 256);
+  if (blocks > sm_count() * 8) blocks = sm_count() * 8;
+  k_pressure64<<<blocks, 256, 0, st>>>(Sig, P, g);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_cfl64(const double *Sig, const double *vR, const double *vp, Ctl *ctl, const Geom64 &g,
