@@ -36,17 +36,6 @@ int dg_handle::fail(int code, const char *what, const char *why) {
   return code;
 }
 
-// e^{-2 pi i j / M}, j < n
-static std::vector<double2> roots_table(int n, int M) {
-  std::vector<double2> r(n);
-  for (int t = 0; t < n; ++t) {
-    long double a = 2.0L * 3.141592653589793238462643383279502884L * (long double)t / (long double)M;
-    r[t].x = (double)cosl(a);
-    r[t].y = (double)-sinl(a);
-  }
-  return r;
-}
-
 template <typename T>
 static cudaError_t dmalloc(T **p, size_t n) {
   return cudaMalloc((void **)p, (n ? n : 1) * sizeof(T));
@@ -66,7 +55,7 @@ static int validate(const dg_params *p, std::string *why) {
   if (p->precision != DG_PREC_FP64 && p->precision != DG_PREC_MIXED) { *why = "precision must be DG_PREC_FP64 or DG_PREC_MIXED"; return DG_ERR_INVALID; }
   if (p->basic_state != DG_BASIC_FFT && p->basic_state != DG_BASIC_ELLIPTIC) { *why = "basic_state must be DG_BASIC_FFT or DG_BASIC_ELLIPTIC"; return DG_ERR_INVALID; }
   FftPlan a, c;
-  if (!make_fft_plan(p->Nphi, &a) || !make_fft_plan(p->Nu, &c)) {
+  if (!make_fft_plan<double2>(p->Nphi, &a) || !make_fft_plan<double2>(p->Nu, &c)) {
     snprintf(b, sizeof b, "Nphi=%d and 2*Nu=%d must factor into 2, 3 and 5", p->Nphi, 2 * p->Nu);
     *why = b;
     return DG_ERR_UNSUPPORTED;
@@ -96,15 +85,20 @@ int dg_handle::init(const dg_params &pp) {
   }
   M = 2 * Nu;
   Nc = Nphi / 2 + 1;
-  make_fft_plan(Nphi, &plPhi);
-  make_fft_plan(Nu, &plU);
   const size_t n = (size_t)Nu * Nphi;
   MK(dmalloc(&dR, Nu)); MK(dmalloc(&dRf, Nu + 1)); MK(dmalloc(&dVol, Nu));
-  MK(dmalloc(&dSqrtR, Nu)); MK(dmalloc(&dR32, Nu));
+  MK(dmalloc(&dPhiScale, Nu)); MK(dmalloc(&dSqrtR, Nu)); MK(dmalloc(&dR32, Nu));
   MK(cudaMemcpy(dR, R.data(), Nu * sizeof(double), cudaMemcpyHostToDevice));
   MK(cudaMemcpy(dRf, Rf.data(), (Nu + 1) * sizeof(double), cudaMemcpyHostToDevice));
   MK(cudaMemcpy(dVol, Vol.data(), Nu * sizeof(double), cudaMemcpyHostToDevice));
-  MK(cudaMemcpy(dSqrtR, sqrtR.data(), Nu * sizeof(double), cudaMemcpyHostToDevice));
+  {
+    // the inverse transforms' normalisation and the potential's factor (kalnajs.hpp:58-62)
+    const double pref = -p.G * du * dphi / (static_cast<double>(M) * Nphi);
+    std::vector<double> ps(Nu);
+    for (int i = 0; i < Nu; ++i) ps[i] = pref / sqrtR[i];
+    MK(cudaMemcpy(dPhiScale, ps.data(), Nu * sizeof(double), cudaMemcpyHostToDevice));
+    MK(cudaMemcpy(dSqrtR, sqrtR.data(), Nu * sizeof(double), cudaMemcpyHostToDevice));
+  }
   MK(cudaMemcpy(dR32, R32.data(), Nu * sizeof(double), cudaMemcpyHostToDevice));
   for (int b = 0; b < 2; ++b) {
     MK(dmalloc(&S[b], n)); MK(dmalloc(&VR[b], n)); MK(dmalloc(&VP[b], n));
@@ -115,28 +109,13 @@ int dg_handle::init(const dg_params &pp) {
   if (p.precision == DG_PREC_FP64 && p.gamma_gas != 2.0)
     for (int b = 0; b < 2; ++b) MK(dmalloc(&PR[b], n));
   MK(dmalloc(&dPhi, n)); MK(dmalloc(&gA, n)); MK(dmalloc(&gB, n));
-  ldW = Nu + (Nu & 1);
-  MK(dmalloc(&W, (size_t)Nc * ldW)); MK(dmalloc(&Khat, (size_t)Nc * M));
-  {
-    // one buffer: stage twiddles of both directions, e^{-2 pi i j / M}, then the positions
-    std::vector<double2> t1, t2, hf = roots_table(Nu, M);
-    std::vector<unsigned short> p1, p2;
-    fft_tables(plPhi, &t1, &p1);
-    fft_tables(plU, &t2, &p2);
-    const size_t n1 = t1.size(), n2 = t2.size(), npos = ((size_t)Nphi + Nu + 7) / 8;
-    std::vector<double2> t(n1 + n2 + Nu + npos);
-    std::copy(t1.begin(), t1.end(), t.begin());
-    std::copy(t2.begin(), t2.end(), t.begin() + n1);
-    std::copy(hf.begin(), hf.end(), t.begin() + n1 + n2);
-    unsigned short *ps = reinterpret_cast<unsigned short *>(t.data() + n1 + n2 + Nu);
-    std::copy(p1.begin(), p1.end(), ps);
-    std::copy(p2.begin(), p2.end(), ps + Nphi);
-    MK(dmalloc(&twPhi, t.size()));
-    MK(cudaMemcpy(twPhi, t.data(), t.size() * sizeof(double2), cudaMemcpyHostToDevice));
-    twU = twPhi + n1;
-    halfU = twU + n2;
-    posPhi = reinterpret_cast<unsigned short *>(halfU + Nu);
-    posU = posPhi + Nphi;
+  products = p.precision == DG_PREC_MIXED && !mixed_fft_grid(Nu, Nphi);
+  if (products) {
+    MK(setup::build(Nu, Nphi, &sg));
+  } else {
+    ldW = Nu + (Nu & 1);
+    MK(dmalloc(&W, (size_t)Nc * ldW)); MK(dmalloc(&Khat, (size_t)Nc * M));
+    MK(build_fft_tables(Nu, Nphi, &ft));
   }
   MK(dmalloc(&scratch, 64));
   MK(dmalloc(&ctl, 1));
@@ -192,13 +171,24 @@ int dg_handle::init(const dg_params &pp) {
 
 // kalnajs.hpp:105-116: khat = r2c of the kernel sampled at wrapped offsets.
 int dg_handle::build_khat() {
+  if (products) {
+    double *tmp = nullptr;
+    MK(dmalloc(&tmp, (size_t)M * p.Nphi));
+    cudaError_t e = launch_kernel_samples64(tmp, M, p.Nphi, du, dphi, p.eps, st);
+    if (e == cudaSuccess) e = setup::khat(tmp, &sg, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    cudaFree(tmp);
+    MK(e);
+    return DG_OK;
+  }
   const size_t ns = (size_t)M * p.Nphi;
   double2 *spec = nullptr;  // the samples' phi spectra [m][p], then the samples
   MK(dmalloc(&spec, (size_t)Nc * M + (ns + 1) / 2));
   double *tmp = reinterpret_cast<double *>(spec + (size_t)Nc * M);
   cudaError_t e = launch_kernel_samples64(tmp, M, p.Nphi, du, dphi, p.eps, st);
-  if (e == cudaSuccess) e = launch_phi_fwd(tmp, M, nullptr, spec, M, plPhi, twPhi, posPhi, st);
-  if (e == cudaSuccess) e = launch_u_khat(spec, M, Nc, plU, twU, halfU, Khat, st);
+  const FftDisk<double2> d{{tmp, tmp}, nullptr, spec, nullptr, nullptr, nullptr};
+  if (e == cudaSuccess) e = launch_phi_fwd<double2>(d, 0, M, M, ft, st);
+  if (e == cudaSuccess) e = launch_u_khat(spec, M, Nc, ft, Khat, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   cudaFree(spec);
   MK(e);
@@ -211,10 +201,11 @@ void dg_handle::release() {
   mixed_release();
   if (graph_exec) cudaGraphExecDestroy(graph_exec);
   if (diag) cudaFree(diag);
-  void *ptrs[] = {rowtab, dR, dRf, dVol, dSqrtR, dR32, S[0], S[1], VR[0], VR[1], VP[0], VP[1], PR[0], PR[1], dPhi, gA, gB,
-                  W, Khat, twPhi, scratch, ctl};
+  void *ptrs[] = {rowtab, dR, dRf, dVol, dPhiScale, dSqrtR, dR32, S[0], S[1], VR[0], VR[1], VP[0], VP[1], PR[0], PR[1], dPhi, gA, gB,
+                  W, Khat, ft.buf, scratch, ctl};
   for (void *q : ptrs)
     if (q) cudaFree(q);
+  setup::release(&sg);
   if (hctl) cudaFreeHost(hctl);
   if (hdt) cudaFreeHost(hdt);
   for (auto &e : ev_pool) cudaEventDestroy(e);
@@ -224,15 +215,20 @@ void dg_handle::release() {
 // ---------------------------------------------------------------------------------
 // gravity (FP64): kalnajs.hpp:48-63
 int dg_handle::potential64(const double *dSig, double *dOut) {
+  if (products) {
+    const double pref = -p.G * du * dphi / (static_cast<double>(M) * p.Nphi);
+    MK(setup::potential(dSig, dR32, pref, dSqrtR, dOut, sg, st));
+    return DG_OK;
+  }
+  const FftDisk<double2> d{{dSig, dSig}, dR32, W, Khat, dPhiScale, dOut};
   MK(prof_begin(DG_PROF_GRAV_PHI_FWD));
-  MK(launch_phi_fwd(dSig, p.Nu, dR32, W, ldW, plPhi, twPhi, posPhi, st));
+  MK(launch_phi_fwd<double2>(d, 0, p.Nu, ldW, ft, st));
   MK(prof_end(DG_PROF_GRAV_PHI_FWD));
   MK(prof_begin(DG_PROF_GRAV_U));
-  MK(launch_u_conv(W, ldW, Nc, plU, twU, halfU, Khat, st));
+  MK(launch_u_conv<double2>(d, Nc, ldW, ft, st));
   MK(prof_end(DG_PROF_GRAV_U));
-  const double pref = -p.G * du * dphi / (static_cast<double>(M) * p.Nphi);
   MK(prof_begin(DG_PROF_GRAV_PHI_INV));
-  MK(launch_phi_inv(W, ldW, p.Nu, plPhi, twPhi, posPhi, pref, dSqrtR, dOut, st));
+  MK(launch_phi_inv<double2>(d, p.Nu, ldW, ft, st));
   MK(prof_end(DG_PROF_GRAV_PHI_INV));
   return DG_OK;
 }

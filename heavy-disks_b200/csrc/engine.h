@@ -8,6 +8,8 @@
 #include "kernels.h"
 
 struct MixedState;  // mixed.cu
+// whether a mixed-precision grid's gravity runs as FP32 FFTs (else the tensor-core products)
+bool mixed_fft_grid(int Nu, int Nphi);
 struct MixedGroup;  // mixed.cu: disks of a batched sweep stepped by one launch per kernel
 struct dg_handle;
 // Grouping key of a disk ("" when it cannot join a group; 1024^2 disks, whose fused
@@ -32,7 +34,7 @@ struct dg_handle {
   double umin = 0, umax = 0, du = 0, dphi = 0;
   int M = 0, Nc = 0;
   std::vector<double> R, Rf, Vol, sqrtR, R32;
-  double *dR = nullptr, *dRf = nullptr, *dVol = nullptr, *dSqrtR = nullptr, *dR32 = nullptr;
+  double *dR = nullptr, *dRf = nullptr, *dVol = nullptr, *dPhiScale = nullptr, *dSqrtR = nullptr, *dR32 = nullptr;
   double *rowtab = nullptr;  // per-row / per-face constants of the FP64 hydro kernel
   dg::Geom64 geom{};
 
@@ -41,15 +43,15 @@ struct dg_handle {
   double *PR[2] = {nullptr, nullptr};  // pressure of S[.] (FP64 path, Gamma != 2)
   int cur = 0;
   double *dPhi = nullptr, *gA = nullptr, *gB = nullptr;
-  // phi half spectra [m][i], row stride ldW (Nu rounded up to even); the real khat table
-  // (fft_smem.cuh k_u_khat, read through
-  // khat_at); stage twiddles, e^{-2 pi i j / 2 Nu} and
-  // frequency positions of the transforms (one buffer, owned by twPhi)
-  double2 *W = nullptr, *twPhi = nullptr, *twU = nullptr, *halfU = nullptr;
+  // phi half spectra [m][i], row stride ldW (Nu rounded up to even), and the real khat table
+  // (fft_smem.cuh k_u_khat)
+  double2 *W = nullptr;
   double *Khat = nullptr;
   int ldW = 0;
-  unsigned short *posPhi = nullptr, *posU = nullptr;
-  dg::FftPlan plPhi{}, plU{};
+  dg::FftTables<double2> ft;
+  // disks on the tensor-core products (their set-up only) use these transforms instead
+  bool products = false;
+  dg::setup::Gravity sg;
   double *scratch = nullptr;  // 64 doubles of reduction output
 
   // control block (device) and a pinned host mirror
@@ -107,6 +109,8 @@ struct dg_handle {
 
   // mixed-precision path (mixed.cu)
   int mixed_init();
+  int mixed_init_fft();
+  int mixed_init_products();
   void mixed_release();
   int mixed_enqueue_step();
   int mixed_enqueue_step_forces(const double *gR, const double *gp);
@@ -116,6 +120,7 @@ struct dg_handle {
   int mixed_upload_state(const double *Sig, const double *vR, const double *vp);
   int mixed_download_state(double *Sig, double *vR, double *vp);
   int mixed_gravity();
+  int mixed_gravity_fft(const dg::FftDisk<float2> &d, int b);
   int mixed_gravity_kernels() const;
   int mixed_hydro_kernels() const;
   int mixed_autotune();

@@ -1,5 +1,5 @@
-// Stage list of one FFT length of the plain (FP64) gravity path, and the layout of its khat
-// table; the kernels are in fft_smem.cuh.
+// Stage list of one FFT length, and what the gravity passes read and write of one disk; the
+// kernels are in fft_smem.cuh and fft_fixed.cuh.
 #pragma once
 
 #include "dg_common.cuh"
@@ -18,12 +18,26 @@ struct FftPlan {
   int tw[kFftMaxStages];                // offset of the stage's twiddles w_L^{j q}, [q - 1][j]
   int threads = 0;                      // threads per transform
   int ntw = 0;                          // entries of the twiddle table
+  bool fixed = false;                   // a length of fft_fixed.cuh, with its radices
 };
 
-// khat(p, m) from that table: posu[q] is where an N-point transform leaves frequency q.
-__device__ __forceinline__ double khat_at(const double *__restrict__ kr, const unsigned short *__restrict__ posu,
-                                          int N, int m, int p) {
-  return kr[((size_t)2 * m + (p & 1)) * N + posu[p >> 1]];
-}
+// One disk's side of the three gravity passes, V = double2 (plain path) or float2 (mixed).
+template <typename V> struct FftDisk {
+  using T = decltype(V::x);
+  const T *src[2];     // the two ping-pong inputs of pass 1
+  const T *inscale;    // per row, or NULL
+  V *W;                // half spectra [m][ldw]
+  const T *kr;         // khat in transform order
+  const T *outscale;   // per row
+  T *out;              // the potential
+};
+
+// Tables of one transform length for both directions of a grid.
+template <typename V> struct FftTables {
+  FftPlan phi, u;
+  V *buf = nullptr;  // owns: stage twiddles of phi and u, e^{-2 pi i j / 2 Nu}, positions
+  const V *twPhi = nullptr, *twU = nullptr, *half = nullptr;
+  const unsigned short *posPhi = nullptr, *posU = nullptr;
+};
 
 }  // namespace dg

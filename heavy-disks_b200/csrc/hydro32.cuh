@@ -36,11 +36,26 @@ struct Rows32 {
   int Nu, Nphi;
   float dphi, inv2dphi, invdu, inv2du, Kpoly, gamma, gmstar;
   int gamma2;  // gamma == 2: P = K Sigma^2 exactly
+  int one_round;  // sigma_new32 in place of two roundings
 };
 
 // hydro.hpp:16-18; a*b > 0 means |a + b| >= max(|a|, |b|) > 0, so the fast divide is safe
 __device__ __forceinline__ float vanleer32(float a, float b) {
   return (a * b > 0.f) ? __fdividef(2.f * a * b, a + b) : 0.f;
+}
+
+// The new sigma from its old value and the increments of both sweeps in one rounding
+// (Rows32::one_round; dsr = sigma_dr32, the radial increment).  On fine grids the radial
+// increment is a few units in the last place of sigma; rounded by itself it errs alike over
+// long stretches of a row and over many steps, which adds up in the total mass: 300 steps of
+// the 4096^2 seed drift by 1.3e-11 with two roundings and by 1.1e-13 with one.  Disks
+// on FFT gravity of 2^21 zones or more take the one.  Smaller ones have coarser increments,
+// and under the tensor-core gravity the noise of its split-BF16 operands (16 times the FFT's)
+// breaks those stretches up; they keep the two, since in a drained edge (see mixed_fft_grid)
+// the last place of sigma is what is left of the density.
+__device__ __forceinline__ float sigma_dr32(float dt, float dF, float iv) { return __fmul_rn(__fmul_rn(dt, dF), iv); }
+__device__ __forceinline__ float sigma_new32(float s, float dsr, float dt, float dF, float iv) {
+  return __fadd_rn(s, __fmaf_rn(__fmul_rn(dt, dF), iv, dsr));
 }
 
 // P(Sigma0 + s) - P(Sigma0) for P = K Sigma^gamma

@@ -93,7 +93,8 @@ __device__ __forceinline__ float up1(float v) { return __shfl_up_sync(0xffffffff
 __device__ __forceinline__ float dn1(float v) { return __shfl_down_sync(0xffffffffu, v, 1); }
 }  // namespace p2
 
-template <bool G2, int FM, bool IN>
+// SX: the step writes the split-BF16 operand of the tensor-core gravity
+template <bool G2, int FM, bool IN, bool SX>
 __device__ __forceinline__ void hydro32p_tile(
     const float *__restrict__ sig, const float *__restrict__ uu, const float *__restrict__ ww,
     const float *__restrict__ Phi, const double *__restrict__ gRin, const double *__restrict__ gpin,
@@ -385,7 +386,8 @@ __device__ __forceinline__ void hydro32p_tile(
       // S4: radial gather
       const F2 sgi = SG[xs], u1i = U1[xu], w1i = W1[xu];
       const F2 s = add(S(S0), sgi);
-      const F2 s2 = fma(mul(S(dt), sub(FF[xf], FF[xf + LF])), S(iv), sgi);
+      const F2 tr = mul(S(dt), sub(FF[xf], FF[xf + LF]));
+      const F2 s2 = fma(tr, S(iv), sgi);
       const F2 sn = add(S(S0), s2);
       const F2 dd = make_float2(sn.x < 1e-10f ? 1e-10f : sn.x, sn.y < 1e-10f ? 1e-10f : sn.y);
       const F2 rdd = rcp(dd);
@@ -427,7 +429,9 @@ __device__ __forceinline__ void hydro32p_tile(
       const F2 fm1 = make_float2(fm.y, dn1(fm.x)), fr1 = make_float2(fr.y, dn1(fr.x)), fg1 = make_float2(fg.y, dn1(fg.x));
       if (outx || outy) {
         const F2 sn2 = sn;
-        F2 s3 = fma(mul(S(dt), sub(fm, fm1)), S(iv), s2);
+        const F2 tp = mul(S(dt), sub(fm, fm1));
+        F2 s3 = fma(tp, S(iv), s2);
+        if (!SX && g.one_round) s3 = add(sgi, fma(tp, S(iv), mul(tr, S(iv))));  // sigma_new32
         const F2 sn3 = add(S(S0), s3);
         const bool flx = sn3.x < 1e-10f, fly = sn3.y < 1e-10f;
         const F2 d = make_float2(flx ? 1e-10f : sn3.x, fly ? 1e-10f : sn3.y);
@@ -436,26 +440,30 @@ __device__ __forceinline__ void hydro32p_tile(
         const F2 w3 = mul(fma(mul(S(dt), sub(fg, fg1)), S(iv), mul(sn2, w2)), rd);
         s3 = make_float2(flx ? 1e-10f - S0 : s3.x, fly ? 1e-10f - S0 : s3.y);
         const size_t q = (size_t)i * Nphi + jc;
-        const float R32 = c2.w;
-        const F2 xr = mul(S(R32), s3);
-        // split-BF16 operand: one packed conversion per plane, the roundings of split_bf16
-        const __nv_bfloat162 h2 = __floats2bfloat162_rn(xr.x, xr.y);
-        const float2 hf = __bfloat1622float2(h2);
-        const __nv_bfloat162 l2 = __floats2bfloat162_rn(xr.x - hf.x, xr.y - hf.y);
         if (outx && outy) {
           *reinterpret_cast<F2 *>(so + q) = s3;
           *reinterpret_cast<F2 *>(uo + q) = u3;
           *reinterpret_cast<F2 *>(wo + q) = w3;
-          *reinterpret_cast<__nv_bfloat162 *>(Sx.hi + q) = h2;
-          *reinterpret_cast<__nv_bfloat162 *>(Sx.lo + q) = l2;
         } else if (outx) {  // one half of the pair is output (tile edges)
           so[q] = s3.x; uo[q] = u3.x; wo[q] = w3.x;
-          Sx.hi[q] = h2.x;
-          Sx.lo[q] = l2.x;
         } else {
           so[q + 1] = s3.y; uo[q + 1] = u3.y; wo[q + 1] = w3.y;
-          Sx.hi[q + 1] = h2.y;
-          Sx.lo[q + 1] = l2.y;
+        }
+        if (SX) {  // one packed conversion per plane, the roundings of split_bf16
+          const F2 xr = mul(S(c2.w), s3);
+          const __nv_bfloat162 h2 = __floats2bfloat162_rn(xr.x, xr.y);
+          const float2 hf = __bfloat1622float2(h2);
+          const __nv_bfloat162 l2 = __floats2bfloat162_rn(xr.x - hf.x, xr.y - hf.y);
+          if (outx && outy) {
+            *reinterpret_cast<__nv_bfloat162 *>(Sx.hi + q) = h2;
+            *reinterpret_cast<__nv_bfloat162 *>(Sx.lo + q) = l2;
+          } else if (outx) {
+            Sx.hi[q] = h2.x;
+            Sx.lo[q] = l2.x;
+          } else {
+            Sx.hi[q + 1] = h2.y;
+            Sx.lo[q + 1] = l2.y;
+          }
         }
         // CFL rate of the new state (hydro.hpp:54-57)
         const F2 scl = make_float2(flx ? 1e-10f : sn3.x, fly ? 1e-10f : sn3.y);
@@ -522,7 +530,7 @@ __device__ __forceinline__ void hydro32p_tile(
 #undef RC
 }
 
-template <bool G2, int FM>
+template <bool G2, int FM, bool SX>
 __global__ void __launch_bounds__(kThreads32t, 4) k_hydro32p(
     const __grid_constant__ CUtensorMap tmS, const __grid_constant__ CUtensorMap tmU,
     const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmP,
@@ -544,10 +552,10 @@ __global__ void __launch_bounds__(kThreads32t, 4) k_hydro32p(
   // (the first CTA barrier inside the tile function orders the set-up before any wait)
   const int i0 = blockIdx.y * kTileI;
   if (i0 >= 3 && i0 + kTileI + 3 <= g.Nu)
-    hydro32p_tile<G2, FM, true>(sig, uu, ww, Phi, gRin, gpin, so, uo, wo, Sx, ctl, g, sm32t, red, bsum, zsum, &tmS,
+    hydro32p_tile<G2, FM, true, SX>(sig, uu, ww, Phi, gRin, gpin, so, uo, wo, Sx, ctl, g, sm32t, red, bsum, zsum, &tmS,
                                 &tmU, &tmW, &tmP, &bar_ld, &bar_rc, early_state != 0);
   else
-    hydro32p_tile<G2, FM, false>(sig, uu, ww, Phi, gRin, gpin, so, uo, wo, Sx, ctl, g, sm32t, red, bsum, zsum, &tmS,
+    hydro32p_tile<G2, FM, false, SX>(sig, uu, ww, Phi, gRin, gpin, so, uo, wo, Sx, ctl, g, sm32t, red, bsum, zsum, &tmS,
                                  &tmU, &tmW, &tmP, &bar_ld, &bar_rc, early_state != 0);
   if (rowpend) rowtile_done(rowpend + blockIdx.y);  // this tile's outputs are written
 }
@@ -583,11 +591,11 @@ __global__ void __launch_bounds__(kThreads32t, 4) k_hydro32p_group(const HydroDi
   const int i0 = blockIdx.y * kTileI;
   // the predecessor (the group's inverse phi product) writes only dPhi: early state loads
   if (i0 >= 3 && i0 + kTileI + 3 <= d.g.Nu)
-    hydro32p_tile<G2, kForcePhi, true>(d.sig[b], d.u[b], d.w[b], d.dPhi, nullptr, nullptr, d.sig[o], d.u[o], d.w[o],
+    hydro32p_tile<G2, kForcePhi, true, true>(d.sig[b], d.u[b], d.w[b], d.dPhi, nullptr, nullptr, d.sig[o], d.u[o], d.w[o],
                                        d.Sx, d.ctl, d.g, sm32t, red, bsum, zsum, &d.tmS[b], &d.tmU[b], &d.tmW[b],
                                        &d.tmP, &bar_ld, &bar_rc, true);
   else
-    hydro32p_tile<G2, kForcePhi, false>(d.sig[b], d.u[b], d.w[b], d.dPhi, nullptr, nullptr, d.sig[o], d.u[o], d.w[o],
+    hydro32p_tile<G2, kForcePhi, false, true>(d.sig[b], d.u[b], d.w[b], d.dPhi, nullptr, nullptr, d.sig[o], d.u[o], d.w[o],
                                         d.Sx, d.ctl, d.g, sm32t, red, bsum, zsum, &d.tmS[b], &d.tmU[b], &d.tmW[b],
                                         &d.tmP, &bar_ld, &bar_rc, true);
 }

@@ -265,7 +265,9 @@ __device__ __forceinline__ void hydro32t_tile(
   }
   __syncthreads();
 
-  // ---- S4: radial gather of rows i0 .. iend-1, columns c in [1, 63) ----
+  // ---- S4: radial gather of rows i0 .. iend-1, columns c in [1, 63).  sigma and its radial
+  // increment stay in registers for S6 (the same thread's points) ----
+  float sg0[kItOut], dsr[kItOut];
 #pragma unroll
   for (int k = 0; k < kItOut; ++k) {
     const int ri = rg + kRowGroups32t * k, i = i0 + ri;
@@ -275,6 +277,8 @@ __device__ __forceinline__ void hydro32t_tile(
       const float S0 = RC(tS0, i);
       const float s = S0 + sgi;
       const float iv = RC(tInvVol, i);
+      sg0[k] = sgi;
+      dsr[k] = sigma_dr32(dt, FF[xf] - FF[xf + kLd32t], iv);
       const float s2 = sgi + dt * (FF[xf] - FF[xf + kLd32t]) * iv;
       const float sn = S0 + s2;
       const float d = (sn < 1e-10f) ? 1e-10f : sn;
@@ -329,6 +333,7 @@ __device__ __forceinline__ void hydro32t_tile(
       const float s2 = SG[x], u2 = U2[x], w2 = W2[x];
       const float sn2 = S0 + s2;
       float s3 = s2 + dt * (PF[xf] - PF[xf + 1]) * iv;
+      if (g.one_round) s3 = sigma_new32(sg0[k], dsr[k], dt, PF[xf] - PF[xf + 1], iv);
       const float sn3 = S0 + s3;
       const float d = (sn3 < 1e-10f) ? 1e-10f : sn3;
       const float u3 = __fdividef(sn2 * u2 + dt * (PR[xf] - PR[xf + 1]) * iv, d);
@@ -336,10 +341,12 @@ __device__ __forceinline__ void hydro32t_tile(
       if (sn3 < 1e-10f) s3 = 1e-10f - S0;  // floor (hydro.hpp:69)
       const size_t q = (size_t)i * Nphi + jc;
       so[q] = s3; uo[q] = u3; wo[q] = w3;
-      const float xr = RC(tR32, i) * s3;
-      const __nv_bfloat16 hx = __float2bfloat16_rn(xr);
-      Sx.hi[q] = hx;
-      Sx.lo[q] = __float2bfloat16_rn(xr - __bfloat162float(hx));
+      if (Sx.hi) {  // the operand of the tensor-core gravity
+        const float xr = RC(tR32, i) * s3;
+        const __nv_bfloat16 hx = __float2bfloat16_rn(xr);
+        Sx.hi[q] = hx;
+        Sx.lo[q] = __float2bfloat16_rn(xr - __bfloat162float(hx));
+      }
       // CFL rate of the new state (hydro.hpp:54-57)
       const float sc_ = (sn3 < 1e-10f) ? 1e-10f : sn3;
       const float cs = sqrtf(G2 ? g.gamma * g.Kpoly * sc_ : g.gamma * g.Kpoly * powf(sc_, g.gamma - 1.f));

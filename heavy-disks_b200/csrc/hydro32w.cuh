@@ -231,13 +231,15 @@ __global__ void __launch_bounds__(kWarps32 * 32) k_hydro32w(
 
     // ---- radial gather of row i = L-3 from faces i (previous) and i+1 (= f) ----
     const int i = L - 3;
-    float s2 = 0.f, u2 = 0.f, w2 = 0.f;
+    float s2 = 0.f, u2 = 0.f, w2 = 0.f, sg0 = 0.f, dsr = 0.f;
     const bool iok = i >= i0 && i < iend;
     if (iok) {
       const float sgi = sg[1], u1i = u1[1], w1i = w1[1];
       const float S0 = RC(cS0, i);
       const float s = S0 + sgi;
       const float iv = RC(cInvVol, i);
+      sg0 = sgi;
+      dsr = sigma_dr32(dt, fF - F, iv);
       s2 = sgi + dt * (fF - F) * iv;
       const float sn = S0 + s2;
       const float d = (sn < 1e-10f) ? 1e-10f : sn;
@@ -282,6 +284,7 @@ __global__ void __launch_bounds__(kWarps32 * 32) k_hydro32w(
         const float S0 = RC(cS0, i);
         const float sn2 = S0 + s2;
         float s3 = s2 + dt * (Fm - Fm_r) * iv;
+        if (g.one_round) s3 = sigma_new32(sg0, dsr, dt, Fm - Fm_r, iv);
         const float sn3 = S0 + s3;
         const float d = (sn3 < 1e-10f) ? 1e-10f : sn3;
         const float u3 = __fdividef(sn2 * u2 + dt * (FRp - FR_r) * iv, d);
@@ -289,10 +292,12 @@ __global__ void __launch_bounds__(kWarps32 * 32) k_hydro32w(
         if (sn3 < 1e-10f) s3 = 1e-10f - S0;  // floor (hydro.hpp:69)
         const int k = i * Nphi + jg;
         so[k] = s3; uo[k] = u3; wo[k] = w3;
-        const float x = RC(cR32, i) * s3;
-        const __nv_bfloat16 hx = __float2bfloat16_rn(x);
-        Sx.hi[k] = hx;
-        Sx.lo[k] = __float2bfloat16_rn(x - __bfloat162float(hx));
+        if (Sx.hi) {  // the operand of the tensor-core gravity
+          const float x = RC(cR32, i) * s3;
+          const __nv_bfloat16 hx = __float2bfloat16_rn(x);
+          Sx.hi[k] = hx;
+          Sx.lo[k] = __float2bfloat16_rn(x - __bfloat162float(hx));
+        }
         // CFL rate of the new state (hydro.hpp:54-57)
         const float sc_ = (sn3 < 1e-10f) ? 1e-10f : sn3;
         const float cs = sqrtf(g.gamma2 ? g.gamma * g.Kpoly * sc_ : g.gamma * g.Kpoly * powf(sc_, g.gamma - 1.f));

@@ -1,5 +1,6 @@
 // Plain-method (FP64) kernels: fused hydro step, CFL reduction, forces, mode sums,
 // Kalnajs kernel samples, and launchers for the shared-memory FFT passes.
+#include <algorithm>
 #include <cmath>
 
 #include "kernels.h"
@@ -318,7 +319,7 @@ __global__ void k_conserved64(const double *__restrict__ Sig, const double *__re
 
 // ---------------------------------------------------------------------------------
 // host launchers
-static int sm_count() {
+int sm_count() {
   static int n = 0;
   if (!n) {
     int dev = 0;
@@ -421,23 +422,30 @@ cudaError_t launch_kernel_samples64(double *out, int M, int Nphi, double du, dou
 // ---------------------------------------------------------------------------------
 // FFT plans and pass launchers.
 
-// Stage radices: the factors 5 and 3 first, then the power of two in radices 8 and 4.  Radix
-// 16 would save a stage of some lengths, but its registers halve the warps per SM, and a
-// stage costs less than the latency those warps hide.
-bool make_fft_plan(int n, FftPlan *pl) {
+// Stage radices: those of fft_fixed.cuh for its lengths; else the factors 5 and 3 first, then
+// the power of two in radices 8 and 4.
+template <typename V> static bool make_plan(int n, FftPlan *pl) {
   *pl = FftPlan{};
   if (n < 1) return false;
   pl->n = n;
-  int e = 0, rest = n;
-  while (rest % 2 == 0) { ++e; rest /= 2; }
   auto add = [&](int R) { pl->R[pl->ns++] = R; };
-  while (rest % 5 == 0) { add(5); rest /= 5; }
-  while (rest % 3 == 0) { add(3); rest /= 3; }
-  if (rest != 1) return false;
-  while (e > 0) {
-    const int k = (e <= 3) ? e : (e == 4 ? 2 : 3);
-    add(1 << k);
-    e -= k;
+  pl->fixed = fixed_length<V>(n);
+  if (pl->fixed) {
+    int R[5];
+    fixed_radices<V>(n, R);
+    for (int r : R)
+      if (r > 1) add(r);
+  } else {
+    int e = 0, rest = n;
+    while (rest % 2 == 0) { ++e; rest /= 2; }
+    while (rest % 5 == 0) { add(5); rest /= 5; }
+    while (rest % 3 == 0) { add(3); rest /= 3; }
+    if (rest != 1) return false;
+    while (e > 0) {
+      const int k = (e <= 3) ? e : (e == 4 ? 2 : 3);
+      add(1 << k);
+      e -= k;
+    }
   }
   if (pl->ns == 0) return false;  // n = 1
   int L = n;
@@ -458,16 +466,20 @@ bool make_fft_plan(int n, FftPlan *pl) {
   pl->threads = T < 1 ? 1 : T;
   return true;
 }
+template <> bool make_fft_plan<double2>(int n, FftPlan *pl) { return make_plan<double2>(n, pl); }
+template <> bool make_fft_plan<float2>(int n, FftPlan *pl) { return make_plan<float2>(n, pl); }
 
 // Host tables of a plan: the stage twiddles and the position of every frequency.
-void fft_tables(const FftPlan &pl, std::vector<double2> *tw, std::vector<unsigned short> *pos) {
-  tw->assign(pl.ntw, make_double2(1.0, 0.0));
+template <typename V>
+void fft_tables(const FftPlan &pl, std::vector<V> *tw, std::vector<unsigned short> *pos) {
+  using T = real_t<V>;
+  tw->assign(pl.ntw, V{});
   for (int s = 0; s < pl.ns; ++s) {
     const int R = pl.R[s], m = pl.m[s], L = R * m;
     for (int q = 1; q < R; ++q)
       for (int j = 0; j < m; ++j) {
         const long double a = -2.0L * 3.141592653589793238462643383279502884L * (long double)(j * q) / (long double)L;
-        (*tw)[pl.tw[s] + (q - 1) * m + j] = make_double2((double)cosl(a), (double)sinl(a));
+        (*tw)[pl.tw[s] + (q - 1) * m + j] = cx<V>((T)cosl(a), (T)sinl(a));
       }
   }
   pos->assign(pl.n, 0);
@@ -481,11 +493,45 @@ void fft_tables(const FftPlan &pl, std::vector<double2> *tw, std::vector<unsigne
   }
 }
 
+// Plans and device tables of an Nu x Nphi grid, in one buffer.
+template <typename V>
+cudaError_t build_fft_tables(int Nu, int Nphi, FftTables<V> *ft) {
+  using T = real_t<V>;
+  if (!make_fft_plan<V>(Nphi, &ft->phi) || !make_fft_plan<V>(Nu, &ft->u)) return cudaErrorInvalidValue;
+  for (const FftPlan *pl : {&ft->phi, &ft->u}) {
+    const cudaError_t e = pl->fixed ? fixed_attrs<V>(pl->n) : cudaSuccess;
+    if (e != cudaSuccess) return e;
+  }
+  std::vector<V> t1, t2;
+  std::vector<unsigned short> p1, p2;
+  fft_tables<V>(ft->phi, &t1, &p1);
+  fft_tables<V>(ft->u, &t2, &p2);
+  const size_t n1 = t1.size(), n2 = t2.size(), per = sizeof(V) / sizeof(unsigned short);
+  std::vector<V> t(n1 + n2 + Nu + ((size_t)Nphi + Nu + per - 1) / per);
+  std::copy(t1.begin(), t1.end(), t.begin());
+  std::copy(t2.begin(), t2.end(), t.begin() + n1);
+  for (int j = 0; j < Nu; ++j) {
+    const long double a = -3.141592653589793238462643383279502884L * (long double)j / (long double)Nu;
+    t[n1 + n2 + j] = cx<V>((T)cosl(a), (T)sinl(a));
+  }
+  unsigned short *ps = reinterpret_cast<unsigned short *>(t.data() + n1 + n2 + Nu);
+  std::copy(p1.begin(), p1.end(), ps);
+  std::copy(p2.begin(), p2.end(), ps + Nphi);
+  cudaError_t e = cudaMalloc((void **)&ft->buf, t.size() * sizeof(V));
+  if (e == cudaSuccess) e = cudaMemcpy(ft->buf, t.data(), t.size() * sizeof(V), cudaMemcpyHostToDevice);
+  ft->twPhi = ft->buf;
+  ft->twU = ft->buf + n1;
+  ft->half = ft->twU + n2;
+  ft->posPhi = reinterpret_cast<const unsigned short *>(ft->half + Nu);
+  ft->posU = ft->posPhi + Nphi;
+  return e;
+}
+
 // Transforms per CTA: up to 4 (their rows share the 128-byte runs of W), while every SM
 // still gets a CTA.
 static int fft_log2_batch(const FftPlan &pl, int count) {
   int lg = 0;
-  while (lg < 2 && (pl.threads << (lg + 1)) <= kFftMaxThreads && (count >> (lg + 1)) >= sm_count()) ++lg;
+  while (lg < 2 && (pl.threads << (lg + 1)) <= kFftMaxThreads && ((count) >> (lg + 1)) >= sm_count()) ++lg;
   return lg;
 }
 
@@ -496,9 +542,13 @@ cudaError_t prepare_fft_kernels() {
   int dev = 0, optin = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-  const void *fns[] = {(const void *)k_phi_fwd<true>, (const void *)k_phi_fwd<false>, (const void *)k_u_conv<true>,
-                       (const void *)k_u_conv<false>, (const void *)k_u_khat, (const void *)k_phi_inv<true>,
-                       (const void *)k_phi_inv<false>};
+  const void *fns[] = {(const void *)k_phi_fwd<double2, true>, (const void *)k_phi_fwd<double2, false>,
+                       (const void *)k_u_conv<double2, true>,  (const void *)k_u_conv<double2, false>,
+                       (const void *)k_phi_inv<double2, true>, (const void *)k_phi_inv<double2, false>,
+                       (const void *)k_phi_fwd<float2, true>,  (const void *)k_phi_fwd<float2, false>,
+                       (const void *)k_u_conv<float2, true>,   (const void *)k_u_conv<float2, false>,
+                       (const void *)k_phi_inv<float2, true>,  (const void *)k_phi_inv<float2, false>,
+                       (const void *)k_u_khat<double2>};
   for (const void *f : fns) {
     cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
     if (e != cudaSuccess) return e;
@@ -510,36 +560,59 @@ cudaError_t prepare_fft_kernels() {
 // Lengths whose tables go to shared memory (the SMT forms).
 static bool fft_smt(int n) { return n <= 512; }
 
-cudaError_t launch_phi_fwd(const double *src, int nrows, const double *rowscale, double2 *W, int ldw,
-                           const FftPlan &pl, const double2 *tws, const unsigned short *pos, cudaStream_t st) {
+template <typename V>
+cudaError_t launch_phi_fwd(const FftDisk<V> &d, int b, int nrows, int ldw,
+                           const FftTables<V> &ft, cudaStream_t st) {
+  const FftPlan &pl = ft.phi;
+  if (pl.fixed && nrows % 2 == 0) return fixed_phi_fwd<V>(pl.n, d, b, nrows, ldw, ft.twPhi, st);
   const int pairs = (nrows + 1) / 2, lg = fft_log2_batch(pl, pairs), nb = 1 << lg;
   const bool smt = fft_smt(pl.n);
-  const size_t sm = ((size_t)nb * fft_pad_len(pl.n) + (smt ? fft_tab_phi(pl.n, pl.ntw) : 0)) * sizeof(double2);
-  return launch_pdl(smt ? k_phi_fwd<true> : k_phi_fwd<false>, dim3((pairs + nb - 1) / nb), dim3(pl.threads, nb), sm,
-                    st, src, nrows, rowscale, W, ldw, pl, tws, pos, lg);
+  const size_t sm = ((size_t)nb * fft_pad_len<V>(pl.n) + (smt ? fft_tab_phi<V>(pl.n, pl.ntw) : 0)) * sizeof(V);
+  return launch_pdl(smt ? k_phi_fwd<V, true> : k_phi_fwd<V, false>, dim3((pairs + nb - 1) / nb),
+                    dim3(pl.threads, nb), sm, st, d, b, nrows, ldw, pl, ft.twPhi, ft.posPhi, lg);
 }
 
-cudaError_t launch_u_conv(double2 *W, int ldw, int Nc, const FftPlan &pl, const double2 *tws, const double2 *half,
-                          const double *kr, cudaStream_t st) {
+template <typename V>
+cudaError_t launch_u_conv(const FftDisk<V> &d, int Nc, int ldw,
+                          const FftTables<V> &ft, cudaStream_t st) {
+  const FftPlan &pl = ft.u;
+  if (pl.fixed) return fixed_u_conv<V>(pl.n, d, Nc, ldw, ft.twU, ft.half, st);
   const bool smt = fft_smt(pl.n);
-  const size_t sm = ((size_t)2 * fft_pad_len(pl.n) + (smt ? fft_tab_u(pl.n, pl.ntw) : 0)) * sizeof(double2);
-  return launch_pdl(smt ? k_u_conv<true> : k_u_conv<false>, dim3(Nc), dim3(pl.threads, 2), sm, st, W, ldw, pl, tws,
-                    half, kr);
+  const size_t sm = ((size_t)2 * fft_pad_len<V>(pl.n) + (smt ? fft_tab_u<V>(pl.n, pl.ntw) : 0)) * sizeof(V);
+  return launch_pdl(smt ? k_u_conv<V, true> : k_u_conv<V, false>, dim3(Nc), dim3(pl.threads, 2), sm, st, d,
+                    ldw, pl, ft.twU, ft.half);
 }
 
-cudaError_t launch_u_khat(const double2 *W, int ldw, int Nc, const FftPlan &pl, const double2 *tws, const double2 *half,
-                          double *kr, cudaStream_t st) {
-  k_u_khat<<<2 * Nc, pl.threads, (size_t)fft_pad_len(pl.n) * sizeof(double2), st>>>(W, ldw, pl, tws, half, kr);
+template <typename V>
+cudaError_t launch_phi_inv(const FftDisk<V> &d, int nrows, int ldw,
+                           const FftTables<V> &ft, cudaStream_t st) {
+  const FftPlan &pl = ft.phi;
+  if (pl.fixed && nrows % 2 == 0) return fixed_phi_inv<V>(pl.n, d, nrows, ldw, ft.twPhi, st);
+  const int pairs = (nrows + 1) / 2, lg = fft_log2_batch(pl, pairs), nb = 1 << lg;
+  const bool smt = fft_smt(pl.n);
+  const size_t sm = ((size_t)nb * fft_pad_len<V>(pl.n) + (smt ? fft_tab_phi<V>(pl.n, pl.ntw) : 0)) * sizeof(V);
+  return launch_pdl(smt ? k_phi_inv<V, true> : k_phi_inv<V, false>, dim3((pairs + nb - 1) / nb),
+                    dim3(pl.threads, nb), sm, st, d, nrows, ldw, pl, ft.twPhi, ft.posPhi, lg);
+}
+
+cudaError_t launch_u_khat(const double2 *W, int ldw, int Nc, const FftTables<double2> &ft, double *kr,
+                          cudaStream_t st) {
+  const FftPlan &pl = ft.u;
+  k_u_khat<double2><<<2 * Nc, pl.threads, (size_t)fft_pad_len<double2>(pl.n) * sizeof(double2), st>>>(
+      W, ldw, pl, ft.twU, ft.half, kr);
   return cudaGetLastError();
 }
 
-cudaError_t launch_phi_inv(const double2 *W, int ldw, int nrows, const FftPlan &pl, const double2 *tws,
-                           const unsigned short *pos, double pref, const double *sqrtR, double *out, cudaStream_t st) {
-  const int pairs = (nrows + 1) / 2, lg = fft_log2_batch(pl, pairs), nb = 1 << lg;
-  const bool smt = fft_smt(pl.n);
-  const size_t sm = ((size_t)nb * fft_pad_len(pl.n) + (smt ? fft_tab_phi(pl.n, pl.ntw) : 0)) * sizeof(double2);
-  return launch_pdl(smt ? k_phi_inv<true> : k_phi_inv<false>, dim3((pairs + nb - 1) / nb), dim3(pl.threads, nb), sm,
-                    st, W, ldw, nrows, pl, tws, pos, pref, sqrtR, out, lg);
-}
+#define DG_FFT_INSTANCES(V)                                                                                        \
+  template cudaError_t build_fft_tables<V>(int, int, FftTables<V> *);                                              \
+  template cudaError_t launch_phi_fwd<V>(const FftDisk<V> &, int, int, int,               \
+                                         const FftTables<V> &, cudaStream_t);                                     \
+  template cudaError_t launch_u_conv<V>(const FftDisk<V> &, int, int, const FftTables<V> &, \
+                                        cudaStream_t);                                                            \
+  template cudaError_t launch_phi_inv<V>(const FftDisk<V> &, int, int,                    \
+                                         const FftTables<V> &, cudaStream_t);
+DG_FFT_INSTANCES(double2)
+DG_FFT_INSTANCES(float2)
+#undef DG_FFT_INSTANCES
 
 }  // namespace dg

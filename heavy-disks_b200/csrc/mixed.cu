@@ -19,6 +19,7 @@
 #include <map>
 #include <mutex>
 #include <string>
+#include <type_traits>
 #include <utility>
 #include <vector>
 
@@ -103,6 +104,13 @@ struct MixedState {
   float2 *twp = nullptr; // W_M^{p2 i1} with padded rows, [64][kUcTwLd]
   CUtensorMap mXin[2], mTb[2], mYk[2], mUb[2], mRB[2], mRA[2], mRGA[2], mRGB[2], mZmn[2];
   bool tables_ready = false;
+  // gravity by FP32 FFTs in shared memory (fft_smem.cuh; mixed_fft_grid): spectra, khat, row
+  // factors (R^{3/2}, then the potential's) and tables
+  bool fft = false;
+  float2 *W32 = nullptr;
+  float *kr32 = nullptr, *rowfac = nullptr;
+  FftTables<float2> ft32;
+  FftDisk<float2> fd{};
   // Nphi = 4096 on grids whose u convolution runs as four passes: both phi transforms in
   // two split-BF16 passes each (64 x 64, four-step) instead of the dense DFT products
   bool phi4096 = false;
@@ -146,17 +154,22 @@ static cudaError_t smem_attrs(const void *fn, size_t bytes) {
 
 // every instantiation of the tiled hydro kernels takes more than 48 KB of shared memory
 static cudaError_t hydro32t_prepare() {
-  const void *fns[] = {(const void *)k_hydro32t<true, kForcePhi>, (const void *)k_hydro32t<false, kForcePhi>,
-                       (const void *)k_hydro32t<true, kForceArrays>, (const void *)k_hydro32t<false, kForceArrays>,
-                       (const void *)k_hydro32t<true, kForceNone>, (const void *)k_hydro32t<false, kForceNone>,
-                       (const void *)k_hydro32p<true, kForcePhi>, (const void *)k_hydro32p<false, kForcePhi>,
-                       (const void *)k_hydro32p<true, kForceArrays>, (const void *)k_hydro32p<false, kForceArrays>,
-                       (const void *)k_hydro32p<true, kForceNone>, (const void *)k_hydro32p<false, kForceNone>};
-  for (int q = 0; q < 12; ++q) {
-    cudaError_t e = smem_attrs(fns[q], q < 6 ? kSmem32t : kSmem32p);
-    if (e != cudaSuccess) return e;
-  }
-  return cudaSuccess;
+  const void *tile[] = {(const void *)k_hydro32t<true, kForcePhi>, (const void *)k_hydro32t<false, kForcePhi>,
+                        (const void *)k_hydro32t<true, kForceArrays>, (const void *)k_hydro32t<false, kForceArrays>,
+                        (const void *)k_hydro32t<true, kForceNone>, (const void *)k_hydro32t<false, kForceNone>};
+  const void *packed[] = {
+      (const void *)k_hydro32p<true, kForcePhi, true>,     (const void *)k_hydro32p<false, kForcePhi, true>,
+      (const void *)k_hydro32p<true, kForceArrays, true>,  (const void *)k_hydro32p<false, kForceArrays, true>,
+      (const void *)k_hydro32p<true, kForceNone, true>,    (const void *)k_hydro32p<false, kForceNone, true>,
+      (const void *)k_hydro32p<true, kForcePhi, false>,    (const void *)k_hydro32p<false, kForcePhi, false>,
+      (const void *)k_hydro32p<true, kForceArrays, false>, (const void *)k_hydro32p<false, kForceArrays, false>,
+      (const void *)k_hydro32p<true, kForceNone, false>,   (const void *)k_hydro32p<false, kForceNone, false>};
+  cudaError_t e = cudaSuccess;
+  for (const void *f : tile)
+    if (e == cudaSuccess) e = smem_attrs(f, kSmem32t);
+  for (const void *f : packed)
+    if (e == cudaSuccess) e = smem_attrs(f, kSmem32p);
+  return e;
 }
 
 // radial-direction layout of the split-BF16 gravity: factored (M = 2 Nu = 64 x Nu/32) when
@@ -263,8 +276,8 @@ __global__ void k_tab_u(SplitBuf Cu, SplitBuf CuT, int Nu) {
   }
 }
 
-// KW[c][p] = (w_p / M) Re khat(p, m(c)), from the FP64 table (khat_at)
-__global__ void k_tab_kw(float *KW, const double *khat, const unsigned short *posu, int Nu, int Nphi) {
+// KW[c][p] = (w_p / M) Re khat(p, m(c)); khat is the FP64 r2c table [m][0..M)
+__global__ void k_tab_kw(float *KW, const double2 *khat, int Nu, int Nphi) {
   const int M = 2 * Nu;
   const size_t n = (size_t)Nphi * M;
   for (size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x) {
@@ -273,7 +286,7 @@ __global__ void k_tab_kw(float *KW, const double *khat, const unsigned short *po
     phi_mode(c, Nphi, m, im);
     int pp = p > Nu ? p - Nu : p;
     double wgt = (p == 0 || p == Nu) ? 1.0 : 2.0;
-    KW[k] = (float)(wgt / M * khat_at(khat, posu, Nu, m, pp));
+    KW[k] = (float)(wgt / M * khat[(size_t)m * M + pp].x);
   }
 }
 
@@ -322,13 +335,13 @@ __global__ void k_tab_cblock(SplitBuf T, int nr, int nk, int L, int sgn) {
 }
 
 // KW2[(m, p2)][(p1, ri)] = Re khat(p2 + 64 p1, m) / M for m <= Nphi/2 (padding modes: 0)
-__global__ void k_tab_kw2(float *KW2, const double *khat, const unsigned short *posu, int nm, int A, int Nphi) {
+__global__ void k_tab_kw2(float *KW2, const double2 *khat, int nm, int A, int Nphi) {
   const int M = 64 * A;
   const size_t n = (size_t)nm * 64 * 2 * A;
   for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (size_t)gridDim.x * blockDim.x) {
     const int row = (int)(q / (2 * A)), col = (int)(q % (2 * A));
     const int m = row >> 6, p2 = row & 63, p1 = col >> 1;
-    KW2[q] = (m <= Nphi / 2) ? (float)(khat_at(khat, posu, M / 2, m, p2 + 64 * p1) / M) : 0.f;
+    KW2[q] = (m <= Nphi / 2) ? (float)(khat[(size_t)m * M + p2 + 64 * p1].x / M) : 0.f;
   }
 }
 
@@ -359,13 +372,12 @@ __global__ void k_tab_phiA(SplitBuf C) {
 
 // KHM[m][p] = Re khat(p, m) / M for m <= Nphi/2 (padding modes: 0); with real_dft_weights
 // also times w_m / Nphi (w = 1 at m = 0 and Nphi/2, else 2), the inverse real DFT's weights
-__global__ void k_tab_khm(float *KHM, const double *khat, const unsigned short *posu, int nm, int M, int Nphi,
-                          bool real_dft_weights) {
+__global__ void k_tab_khm(float *KHM, const double2 *khat, int nm, int M, int Nphi, bool real_dft_weights) {
   const size_t n = (size_t)nm * M;
   for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (size_t)gridDim.x * blockDim.x) {
     const int m = (int)(q / M);
     const double w = !real_dft_weights ? 1.0 : ((m == 0 || 2 * m == Nphi) ? 1.0 : 2.0) / Nphi;
-    KHM[q] = (m <= Nphi / 2) ? (float)(khat_at(khat, posu, M / 2, m, (int)(q % M)) / M * w) : 0.f;
+    KHM[q] = (m <= Nphi / 2) ? (float)(khat[q].x / M * w) : 0.f;
   }
 }
 
@@ -403,10 +415,12 @@ __global__ void k_to_pert(const double *S, const double *vR, const double *vp, f
     sig[k] = s;
     u[k] = (float)vR[k];
     w[k] = (float)(vp[k] - g.V0d[i]);
-    float x = g.R32[i] * s;
-    __nv_bfloat16 h = __float2bfloat16_rn(x);
-    Sx.hi[k] = h;
-    Sx.lo[k] = __float2bfloat16_rn(x - __bfloat162float(h));
+    if (Sx.hi) {
+      float x = g.R32[i] * s;
+      __nv_bfloat16 h = __float2bfloat16_rn(x);
+      Sx.hi[k] = h;
+      Sx.lo[k] = __float2bfloat16_rn(x - __bfloat162float(h));
+    }
   }
 }
 
@@ -430,6 +444,24 @@ __global__ void k_full_to_sx(const double *S, SplitBuf Sx, const double *R32d, i
     __nv_bfloat16 h = __float2bfloat16_rn(x);
     Sx.hi[k] = h;
     Sx.lo[k] = __float2bfloat16_rn(x - __bfloat162float(h));
+  }
+}
+
+// the same in FP32, the FFT gravity's input
+__global__ void k_full_to_f32(const double *S, float *x, const double *R32d, int Nu, int Nphi) {
+  const size_t n = (size_t)Nu * Nphi;
+  for (size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x)
+    x[k] = (float)(R32d[k / Nphi] * S[k]);
+}
+
+// khat in the FP32 transforms' order, from the FP64 table (rows (m, parity))
+__global__ void k_tab_kr32(float *kr32, const double *khat, const unsigned short *pos32, const unsigned short *pos64,
+                           int N, int rows) {
+  const size_t n = (size_t)rows * N;
+  for (size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x) {
+    const size_t row = k / N;
+    const int q = (int)(k % N);
+    kr32[row * N + pos32[q]] = (float)khat[row * N + pos64[q]];
   }
 }
 
@@ -576,15 +608,6 @@ static void free_split(SplitBuf &b) {
 // 128 x 128 or (where N is a multiple of 256) 128 x 256 tiles
 constexpr int kPersist = 8, kPersistWide = 16;
 
-// SMs of the current device (the persistent products' grid)
-static int sm_count() {
-  int dev = 0, n = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-      n <= 0)
-    n = 148;
-  return n;
-}
-
 // gemm(): one split-BF16 product.  ns = pipeline stages of the tile kernel (1, 2 or 4; 0
 // picks by K), or kPersist for the persistent kernel.
 template <int MODE, bool A_MN = false, bool B_MN = false>
@@ -646,45 +669,42 @@ static cudaError_t prepare_gemm() {
   return smem_attrs((const void *)tc::k_gemm_split<MODE, A_MN, B_MN, tc::STAGES>, tc::smem_bytes(tc::STAGES));
 }
 
-int dg_handle::mixed_init() {
-  const int Nu = p.Nu, Nphi = p.Nphi;
-  if (Nu % tc::BM || Nphi % tc::BM) {
-    char b[160];
-    snprintf(b, sizeof b, "Nu=%d Nphi=%d: the tensor-core gravity needs multiples of %d", Nu, Nphi, tc::BM);
-    return fail(DG_ERR_UNSUPPORTED, "mixed precision", b);
-  }
-  if (!encode_fn()) return fail(DG_ERR_UNSUPPORTED, "mixed precision", "cuTensorMapEncodeTiled unavailable");
-  mx = new MixedState();
+// FP32 FFT gravity: spectra, khat and factors of the handle, tables of the grid
+int dg_handle::mixed_init_fft() {
   MixedState &X = *mx;
-  X.Nu = Nu;
-  X.Nphi = Nphi;
-  const size_t n = (size_t)Nu * Nphi;
-  for (int b = 0; b < 2; ++b) {
-    XK(dalloc(&X.sig[b], n)); XK(dalloc(&X.u[b], n)); XK(dalloc(&X.w[b], n));
+  const int Nu = p.Nu, Nphi = p.Nphi;
+  XK(build_fft_tables(Nu, Nphi, &X.ft32));
+  XK(dalloc(&X.W32, (size_t)Nc * Nu));
+  XK(dalloc(&X.kr32, (size_t)Nc * M));
+  XK(dalloc(&X.rowfac, (size_t)2 * Nu));
+  std::vector<float> f((size_t)2 * Nu);
+  for (int i = 0; i < Nu; ++i) {
+    f[i] = (float)R32[i];
+    f[Nu + i] = (float)(-p.G * du * dphi / ((double)M * Nphi) / sqrtR[i]);
   }
+  XK(cudaMemcpy(X.rowfac, f.data(), f.size() * sizeof(float), cudaMemcpyHostToDevice));
+  k_tab_kr32<<<grid_for((size_t)Nc * M), 256, 0, st>>>(X.kr32, Khat, X.ft32.posU, ft.posU, Nu, 2 * Nc);
+  XK(cudaGetLastError());
+  X.fd = FftDisk<float2>{{X.sig[0], X.sig[1]}, X.rowfac, X.W32, X.kr32, X.rowfac + Nu, X.dPhi};
+  return DG_OK;
+}
+
+// tensor-core gravity: operands, DFT tables and tensor maps of the products
+int dg_handle::mixed_init_products() {
+  MixedState &X = *mx;
+  const int Nu = p.Nu, Nphi = p.Nphi;
+  const size_t n = (size_t)Nu * Nphi;
   XK(alloc_split(X.Sx, n)); XK(alloc_split(X.X1, n)); XK(alloc_split(X.Z, n));
   XK(alloc_split(X.Wt, (size_t)Nphi * 2 * Nu));
   XK(alloc_split(X.Fphi, (size_t)Nphi * Nphi)); XK(alloc_split(X.Gphi, (size_t)Nphi * Nphi));
   XK(alloc_split(X.Cu, (size_t)2 * Nu * Nu)); XK(alloc_split(X.CuT, (size_t)2 * Nu * Nu));
   XK(dalloc(&X.KW, (size_t)Nphi * 2 * Nu));
-  XK(dalloc(&X.dPhi, n));
-  static_assert(kTileI == tc::kPfHydroRows && kTileI % tc::kPfRows == 0, "row tiles of the hand-over");
-  XK(dalloc(&X.rowpend, (size_t)(Nu + kTileI - 1) / kTileI));
-  {
-    const char *rs = getenv("DISKGPU_ROWSYNC");
-    X.rowsync = !(rs && strcmp(rs, "0") == 0);
-  }
-  XK(cudaMemsetAsync(X.rowpend, 0, (size_t)(Nu + kTileI - 1) / kTileI * sizeof(int), st));
   XK(dalloc(&X.phiscale, Nu));
-  XK(dalloc(&X.rowbuf, (size_t)24 * (Nu + 1)));
-  XK(dalloc(&X.rowtab, (size_t)(Nu + kRowTabExtra) * kRowTabW));
-  XK(dalloc(&X.rowbufd, (size_t)4 * Nu));
-  // DFT tables
   k_tab_phi<<<grid_for((size_t)Nphi * Nphi), 256, 0, st>>>(X.Fphi, X.Gphi, Nphi);
   XK(cudaGetLastError());
   k_tab_u<<<grid_for((size_t)2 * Nu * Nu), 256, 0, st>>>(X.Cu, X.CuT, Nu);
   XK(cudaGetLastError());
-  k_tab_kw<<<grid_for((size_t)Nphi * 2 * Nu), 256, 0, st>>>(X.KW, Khat, posU, Nu, Nphi);
+  k_tab_kw<<<grid_for((size_t)Nphi * 2 * Nu), 256, 0, st>>>(X.KW, sg.khat, Nu, Nphi);
   XK(cudaGetLastError());
   std::vector<float> ps(Nu);
   for (int i = 0; i < Nu; ++i) ps[i] = (float)(-p.G * du * dphi / sqrtR[i]);
@@ -721,7 +741,7 @@ int dg_handle::mixed_init() {
     k_tab_cblock<<<64, 256, 0, st>>>(X.RA, A, A, A, -1);       // W_A^{p1 i1}
     k_tab_cblock<<<64, 256, 0, st>>>(X.RGA, A, A, A, +1);      // W_A^{-i1 p1}
     k_tab_cblock<<<64, 256, 0, st>>>(X.RGB, 32, 64, 64, +1);   // W_64^{-i2 p2}
-    k_tab_kw2<<<grid_for((size_t)nm * 128 * A), 256, 0, st>>>(X.KW2, Khat, posU, nm, A, Nphi);
+    k_tab_kw2<<<grid_for((size_t)nm * 128 * A), 256, 0, st>>>(X.KW2, sg.khat, nm, A, Nphi);
     k_tab_tw<<<64, 256, 0, st>>>(X.tw, A, A);
     XK(cudaGetLastError());
     X.fused_u = u_fused(Nu);
@@ -730,7 +750,7 @@ int dg_handle::mixed_init() {
       XK(dalloc(&X.khm, (size_t)nm * 64 * A));
       XK(dalloc(&X.twp, (size_t)64 * tc::kUcTwLd));
       k_tab_tw<<<64, 256, 0, st>>>(X.twp, A, tc::kUcTwLd);
-      k_tab_khm<<<grid_for((size_t)nm * 64 * A), 256, 0, st>>>(X.khm, Khat, posU, nm, 64 * A, Nphi, X.fused_phi);
+      k_tab_khm<<<grid_for((size_t)nm * 64 * A), 256, 0, st>>>(X.khm, sg.khat, nm, 64 * A, Nphi, X.fused_phi);
       XK(cudaGetLastError());
       XK(smem_attrs((const void *)tc::k_uconv, tc::kUcSmem));
     }
@@ -813,6 +833,56 @@ int dg_handle::mixed_init() {
   XK((prepare_gemm<tc::kEpiSplit, false, false>()));
   XK((prepare_gemm<tc::kEpiSplitScaled, false, false>()));
   XK((prepare_gemm<tc::kEpiRowScaleF32, false, false>()));
+  return DG_OK;
+}
+
+// FFTs win on every grid but 1024^2 (step in us, products -> FFT: 256^2 33.9 -> 16.7,
+// 512^2 49 -> 21, 2048 x 1024 135 -> 67, 4096^2 976 -> 519; at 1024^2 the fused transforms take
+// 46.5, FFTs 62).  Up to 2^20 zones a disk stays on the products all the same: runs there take
+// the disk's edge down to 1e-8 of its peak density, where FP32 leaves the velocities to
+// last-place noise, and any other rounding of the gravity draws that noise anew, past 2e-5 of
+// the earlier results (32 sweep disks to t = 0.5: up to 2e-4 of a disk's radial velocity; the
+// grids above, over as much work, stay within 6e-6).  DISKGPU_STAGES asks for the products.
+bool mixed_fft_grid(int Nu, int Nphi) {
+  const char *sv = getenv("DISKGPU_STAGES");
+  return (size_t)Nu * Nphi > 1024 * 1024 && !(sv && *sv);
+}
+
+int dg_handle::mixed_init() {
+  const int Nu = p.Nu, Nphi = p.Nphi;
+  if (Nu % tc::BM || Nphi % tc::BM) {
+    char b[160];
+    snprintf(b, sizeof b, "Nu=%d Nphi=%d: the tensor-core gravity needs multiples of %d", Nu, Nphi, tc::BM);
+    return fail(DG_ERR_UNSUPPORTED, "mixed precision", b);
+  }
+  if (!encode_fn()) return fail(DG_ERR_UNSUPPORTED, "mixed precision", "cuTensorMapEncodeTiled unavailable");
+  mx = new MixedState();
+  MixedState &X = *mx;
+  X.Nu = Nu;
+  X.Nphi = Nphi;
+  const size_t n = (size_t)Nu * Nphi;
+  for (int b = 0; b < 2; ++b) {
+    XK(dalloc(&X.sig[b], n)); XK(dalloc(&X.u[b], n)); XK(dalloc(&X.w[b], n));
+  }
+  X.fft = !products;
+  XK(dalloc(&X.dPhi, n));
+  static_assert(kTileI == tc::kPfHydroRows && kTileI % tc::kPfRows == 0, "row tiles of the hand-over");
+  XK(dalloc(&X.rowpend, (size_t)(Nu + kTileI - 1) / kTileI));
+  {
+    const char *rs = getenv("DISKGPU_ROWSYNC");
+    X.rowsync = !(rs && strcmp(rs, "0") == 0);
+  }
+  XK(cudaMemsetAsync(X.rowpend, 0, (size_t)(Nu + kTileI - 1) / kTileI * sizeof(int), st));
+  XK(dalloc(&X.rowbuf, (size_t)24 * (Nu + 1)));
+  XK(dalloc(&X.rowtab, (size_t)(Nu + kRowTabExtra) * kRowTabW));
+  XK(dalloc(&X.rowbufd, (size_t)4 * Nu));
+  if (X.fft) {
+    int rc = mixed_init_fft();
+    if (rc) return rc;
+  } else {
+    int rc = mixed_init_products();
+    if (rc) return rc;
+  }
   XK(cudaStreamSynchronize(st));
   {
     const char *hk = getenv("DISKGPU_HYDRO32");
@@ -863,7 +933,7 @@ void dg_handle::mixed_release() {
                       &X.IA, &X.IB, &X.Zt, &X.PhA1, &X.PhB2f, &X.PhB1i, &X.PhB2i, &X.PhT, &X.PhX, &X.PhV};
   for (SplitBuf *b : bufs) free_split(*b);
   void *ptrs[] = {X.KW,  X.dPhi, X.rowpend, X.phiscale, X.rowbuf, X.rowtab, X.rowbufd,
-                  X.KW2, X.tw,   X.khm,     X.twp,      X.twphi,  X.twph};
+                  X.KW2, X.tw,   X.khm,     X.twp,      X.twphi,  X.twph, X.W32, X.kr32, X.rowfac, X.ft32.buf};
   for (void *q : ptrs)
     if (q) cudaFree(q);
   delete mx;
@@ -989,6 +1059,7 @@ static int build_basic(dg_handle *h, const double *Sig, const double *vp) {
   g.invdu = (float)(1.0 / h->du); g.inv2du = (float)(1.0 / (2.0 * h->du));
   g.Kpoly = (float)K; g.gamma = (float)gam; g.gmstar = (float)p.gmstar;
   g.gamma2 = (gam == 2.0) ? 1 : 0;
+  g.one_round = (X.fft && (size_t)Nu * Nphi >= (size_t)1 << 21) ? 1 : 0;
   return DG_OK;
 }
 
@@ -1032,13 +1103,17 @@ int dg_handle::mixed_upload_state(const double *Sig, const double *vRh, const do
 // never inside a stream capture) it times the step's kernel variants on the handle's own
 // buffers and keeps the fastest:
 //   * the pipeline depth (1, 2 or 4 stages) of every gravity product, one product at a time
-//     with the others fixed, timing the whole gravity of the uploaded state;
-//   * the hydro form (tiled, packed two-column, warp-marching), writing the other ping-pong
-//     buffers and a scratch control block, so the handle's dt, time and records are untouched.
+//     with the others fixed, timing the whole gravity of the uploaded state (FFT gravity and
+//     the fused transforms have none to choose);
+//   * the hydro form (packed two-column, tiled, warp-marching), each in whole steps on the
+//     other ping-pong buffers and a scratch control block, so the handle's dt, time and
+//     records are untouched.  Timed alone the packed and tiled forms differ by less than the
+//     noise, and on some grids the tiled one was picked and cost 2 to 4 us of a 22 us step.
 // A variant must beat the current choice by 2 % to replace it.  Choices are cached per
 // process by (Nu, Nphi, Gamma = 2, self-gravity), so the disks of a batch that share a grid
 // are tuned once.  DISKGPU_TUNE=0 keeps the defaults (packed hydro, stages by K);
-// DISKGPU_HYDRO32 fixes the hydro form.
+// DISKGPU_HYDRO32 fixes the hydro form; DISKGPU_STAGES asks for the tensor-core products with
+// the given depths.
 namespace {
 struct TuneKey {
   int Nu, Nphi, g2, sg;
@@ -1133,6 +1208,12 @@ int dg_handle::mixed_autotune() {
         snprintf(buf, sizeof buf, " %d", X.ns[k]);
         info += buf;
       }
+    } else if (p.selfgrav && X.fft) {
+      float t;
+      cudaError_t e = time_us([&](bool) -> cudaError_t { return mixed_gravity() ? cudaErrorUnknown : cudaSuccess; }, &t);
+      if (e != cudaSuccess) { rc = fail(DG_ERR_CUDA, "autotune", cudaGetErrorString(e)); break; }
+      snprintf(buf, sizeof buf, "gravity by FP32 FFT %.1f us", t);
+      info += buf;
     } else if (p.selfgrav) {
       // products that run as k_gemm_split (the fused kernels have no pipeline to tune)
       const std::vector<int> slots = !X.factored ? std::vector<int>{0, 1, 2, 5}
@@ -1173,15 +1254,16 @@ int dg_handle::mixed_autotune() {
       h0.fixed_dt = 1;
       const int fm = p.selfgrav ? kForcePhi : kForceNone;
       const int c = cur, o = cur ^ 1;
+      const int steps = (size_t)p.Nu * p.Nphi >= 1024 * 1024 ? 2 : 8;
       auto hyd = [&](bool) -> cudaError_t {
         cudaError_t e = cudaMemcpyAsync(sctl, &h0, sizeof(Ctl), cudaMemcpyHostToDevice, st);
-        if (e != cudaSuccess) return e;
-        return launch_hydro32(X, X.sig[c], X.u[c], X.w[c], X.dPhi, nullptr, nullptr, fm, X.sig[o], X.u[o], X.w[o],
-                              sctl, st);
+        for (int k = 0; k < steps && e == cudaSuccess; ++k) {
+          if (p.selfgrav && mixed_gravity()) return cudaErrorUnknown;
+          e = launch_hydro32(X, X.sig[c], X.u[c], X.w[c], X.dPhi, nullptr, nullptr, fm, X.sig[o], X.u[o], X.w[o],
+                             sctl, st, nullptr, fm == kForcePhi);
+        }
+        return e;
       };
-      // the packed form first: it is timed alone here, but inside a step its TMA-staged tile,
-      // bulk-copied row constants and early control loads overlap the kernels around it, so
-      // another form must beat it by the margin alone
       const int kinds[3] = {MixedState::kHydroPacked, MixedState::kHydroTile, MixedState::kHydroWarp};
       float tk[3] = {0.f, 0.f, 0.f};
       int best = MixedState::kHydroPacked;
@@ -1190,6 +1272,7 @@ int dg_handle::mixed_autotune() {
       for (int q = 0; q < 3 && e == cudaSuccess; ++q) {
         X.hydro_kind = kinds[q];
         e = time_us(hyd, &tk[q]);
+        tk[q] /= steps;
         if (e == cudaSuccess && (q == 0 || tk[q] < 0.98f * tb)) {
           tb = tk[q];
           best = kinds[q];
@@ -1197,7 +1280,7 @@ int dg_handle::mixed_autotune() {
       }
       X.hydro_kind = best;
       if (e != cudaSuccess) { rc = fail(DG_ERR_CUDA, "autotune", cudaGetErrorString(e)); break; }
-      snprintf(buf, sizeof buf, "%shydro %s (packed %.1f us, tile %.1f us, warp %.1f us)", info.empty() ? "" : "; ",
+      snprintf(buf, sizeof buf, "%shydro %s (step with packed %.1f us, tile %.1f us, warp %.1f us)", info.empty() ? "" : "; ",
                kHydroNames[best], tk[0], tk[1], tk[2]);
       info += buf;
     } else {
@@ -1269,9 +1352,14 @@ static cudaError_t launch_hydro32(MixedState &X, const float *sig, const float *
                      gR, gp, so, uo, wo, sx, ctl, X.rows, rowpend, early_state ? 1 : 0);
     };
     const bool g2 = X.rows.gamma2 != 0;
-    if (fm == kForcePhi) g2 ? go(k_hydro32p<true, kForcePhi>) : go(k_hydro32p<false, kForcePhi>);
-    else if (fm == kForceArrays) g2 ? go(k_hydro32p<true, kForceArrays>) : go(k_hydro32p<false, kForceArrays>);
-    else g2 ? go(k_hydro32p<true, kForceNone>) : go(k_hydro32p<false, kForceNone>);
+    auto pick = [&](auto sxc) {
+      constexpr bool SX = decltype(sxc)::value;
+      if (fm == kForcePhi) g2 ? go(k_hydro32p<true, kForcePhi, SX>) : go(k_hydro32p<false, kForcePhi, SX>);
+      else if (fm == kForceArrays) g2 ? go(k_hydro32p<true, kForceArrays, SX>) : go(k_hydro32p<false, kForceArrays, SX>);
+      else g2 ? go(k_hydro32p<true, kForceNone, SX>) : go(k_hydro32p<false, kForceNone, SX>);
+    };
+    if (sx.hi) pick(std::true_type{});
+    else pick(std::false_type{});
     if (e == cudaSuccess && finalize) e = launch_finalize(X, ctl, st);
     return e;
   }
@@ -1299,10 +1387,26 @@ static cudaError_t launch_hydro32(MixedState &X, const float *sig, const float *
 }
 
 
-// dPhi = gravity of s (the split operand in X.Sx)
+// dPhi = gravity of d.src[b] by FP32 FFTs
+int dg_handle::mixed_gravity_fft(const FftDisk<float2> &d, int b) {
+  MixedState &X = *mx;
+  XK(prof_begin(DG_PROF_GRAV_PHI_FWD));
+  XK(launch_phi_fwd<float2>(d, b, p.Nu, p.Nu, X.ft32, st));
+  XK(prof_end(DG_PROF_GRAV_PHI_FWD));
+  XK(prof_begin(DG_PROF_GRAV_U));
+  XK(launch_u_conv<float2>(d, Nc, p.Nu, X.ft32, st));
+  XK(prof_end(DG_PROF_GRAV_U));
+  XK(prof_begin(DG_PROF_GRAV_PHI_INV));
+  XK(launch_phi_inv<float2>(d, p.Nu, p.Nu, X.ft32, st));
+  XK(prof_end(DG_PROF_GRAV_PHI_INV));
+  return DG_OK;
+}
+
+// dPhi = gravity of the current perturbation (or of the split operand in X.Sx)
 int dg_handle::mixed_gravity() {
   MixedState &X = *mx;
   const int Nu = p.Nu, Nphi = p.Nphi;
+  if (X.fft) return mixed_gravity_fft(X.fd, cur);
   tc::GemmArgs a{};
   a.status = &ctl->status;
   if (X.factored) {
@@ -1423,6 +1527,7 @@ int dg_handle::mixed_hydro_kernels() const {
 }
 
 int dg_handle::mixed_gravity_kernels() const {
+  if (mx && mx->fft) return 3;
   if (!u_factored(p.Nu)) return 4;
   if (mx && mx->phi4096) return 8;
   return u_fused(p.Nu) ? 3 : 6;
@@ -1530,6 +1635,20 @@ int dg_handle::mixed_conserved_launch(double *out2) {
 int dg_handle::mixed_potential(const double *dSig, double *dOut) {
   MixedState &X = *mx;
   const size_t n = (size_t)p.Nu * p.Nphi;
+  if (X.fft) {
+    // the idle ping-pong buffer holds the scaled field; the next step overwrites it anyway
+    float *x = X.sig[cur ^ 1];
+    k_full_to_f32<<<grid_for(n), 256, 0, st>>>(dSig, x, dR32, p.Nu, p.Nphi);
+    XK(cudaGetLastError());
+    FftDisk<float2> d = X.fd;
+    d.src[0] = d.src[1] = x;
+    d.inscale = nullptr;
+    int rc = mixed_gravity_fft(d, 0);
+    if (rc) return rc;
+    k_f32_to_f64<<<grid_for(n), 256, 0, st>>>(X.dPhi, dOut, n);
+    XK(cudaGetLastError());
+    return DG_OK;
+  }
   k_full_to_sx<<<grid_for(n), 256, 0, st>>>(dSig, X.Sx, dR32, p.Nu, p.Nphi);
   XK(cudaGetLastError());
   int rc = mixed_gravity();
@@ -1577,6 +1696,7 @@ std::string mixed_group_key(const dg_handle *h, bool with_fused) {
   const MixedState &X = *h->mx;
   // dense products, or the fused 1024^2 transforms (the other factored forms step alone)
   if (X.factored && (!X.fused_phi || !with_fused)) return std::string();
+  if (X.fft) return std::string();  // large enough to fill the GPU alone
   if (X.hydro_kind != MixedState::kHydroPacked && X.hydro_kind != MixedState::kHydroTile) return std::string();
   char b[160];
   snprintf(b, sizeof b, "%d:%d:%d:%d:%d:%d:%d,%d,%d,%d", h->dev, X.Nu, X.Nphi, X.fused_phi ? 1 : 0, X.rows.gamma2,
@@ -1630,7 +1750,7 @@ static int group_launch(MixedGroup *g, cudaStream_t st, bool prepare) {
   dg_handle *L = g->lead;
   MixedState &X = *L->mx;
   const int Nu = X.Nu, Nphi = X.Nphi, G = (int)g->disks.size();
-  cudaError_t e;
+  cudaError_t e = cudaSuccess;
   if (g->fused) {
     // phi transform -> Xin, u convolution (F1 F2 I1 I2) -> Zt, inverse phi transform -> dPhi
     if (prepare) {
@@ -1653,9 +1773,10 @@ static int group_launch(MixedGroup *g, cudaStream_t st, bool prepare) {
   }
   // G1: X1[c][i] = Fphi[c][:] . Sx[i][:];  G2: Wt[c][p] = KW[c][p] X1[c][:] . Cu[p][:];
   // G3: Z[i][c] = CuT[i][:] . Wt[c][:];    G4: dPhi[i][j] = phiscale[i] Z[i][:] . Gphi[j][:]
-  if (!g->fused) e = gemm_group<tc::kEpiSplit, false, false, false>(X.mFphi[0], X.mFphi[1], g->gd[0], G, Nphi, Nu, Nphi, st, g->ns[0],
+  const bool dense = !g->fused;
+  if (dense) e = gemm_group<tc::kEpiSplit, false, false, false>(X.mFphi[0], X.mFphi[1], g->gd[0], G, Nphi, Nu, Nphi, st, g->ns[0],
                                                        prepare, g->persist, g->nsm);
-  if (!g->fused) {
+  if (dense) {
   if (e != cudaSuccess) return L->fail(DG_ERR_CUDA, "batch group: phi DFT", cudaGetErrorString(e));
   e = gemm_group<tc::kEpiSplitScaled, false, false, true>(X.mCu[0], X.mCu[1], g->gd[1], G, Nphi, 2 * Nu, Nu, st,
                                                           g->ns[1], prepare, g->persist, g->nsm);
@@ -1668,8 +1789,8 @@ static int group_launch(MixedGroup *g, cudaStream_t st, bool prepare) {
   if (e != cudaSuccess) return L->fail(DG_ERR_CUDA, "batch group: inverse phi DFT", cudaGetErrorString(e));
   }
   const bool packed = g->kind == MixedState::kHydroPacked;
-  auto hk = packed ? (g->g2 ? k_hydro32p_group<true> : k_hydro32p_group<false>)
-                   : (g->g2 ? k_hydro32t_group<true> : k_hydro32t_group<false>);
+  auto hp = g->g2 ? k_hydro32p_group<true> : k_hydro32p_group<false>;
+  auto hk = packed ? hp : (g->g2 ? k_hydro32t_group<true> : k_hydro32t_group<false>);
   const size_t hsm = packed ? kSmem32p : kSmem32t;
   if (prepare) {
     e = smem_attrs((const void *)hk, hsm);
