@@ -23,6 +23,7 @@
 #include <vector>
 
 #include "diskgpu.h"
+#include "kernels.h"
 #include "tc_gemm.cuh"
 
 // mixed.cu: a K-major BF16 tensor map of a [rows][cols] matrix, 64-column boxes of box_rows rows
@@ -48,6 +49,8 @@ __device__ __forceinline__ void put_split(Split s, size_t k, float v) {
 // input rows -> split operand [rows][P], zero beyond n rows and n_in columns
 __global__ void k_x_to_split(int n, int n_in, int P, int rows, const float *__restrict__ x, Split X) {
   const int cnt = rows * P;
+  dg::pdl_wait();
+  dg::pdl_trigger();
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < cnt; k += gridDim.x * blockDim.x) {
     const int b = k / P, i = k - b * P;
     put_split(X, k, (b < n && i < n_in) ? x[(size_t)b * n_in + i] : 0.f);
@@ -61,6 +64,8 @@ __global__ void k_mse(int n, int n_out, int P, int rows, float inv, const float 
   __shared__ float red[256];
   float s = 0.f;
   const int cnt = rows * P;
+  dg::pdl_wait();
+  dg::pdl_trigger();
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < cnt; k += gridDim.x * blockDim.x) {
     const int b = k / P, o = k - b * P;
     const float d = (b < n && o < n_out) ? Y[k] - T[(size_t)b * n_out + o] : 0.f;
@@ -83,6 +88,8 @@ __global__ void k_colsum(int B, int ld, const float *__restrict__ dZ, float *__r
   __shared__ float red[256];
   const int j = blockIdx.x;
   float s = 0.f;
+  dg::pdl_wait();
+  dg::pdl_trigger();
   for (int b = threadIdx.x; b < B; b += blockDim.x) s += dZ[(size_t)b * ld + j];
   red[threadIdx.x] = s;
   __syncthreads();
@@ -230,8 +237,8 @@ static cudaError_t product_ns(cudaStream_t st, const CUtensorMap *a2, const CUte
                               int M, int N, int K, const GemmArgs &args, bool prepare) {
   auto kern = tc::k_gemm_split<MODE, A_MN, B_MN, NS>;
   if (prepare) return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc::smem_bytes(NS));
-  kern<<<dim3(N / tc::BN, M / tc::BM), tc::kThreads, tc::smem_bytes(NS), st>>>(a2[0], a2[1], bh, bl, args);
-  return cudaGetLastError();
+  return dg::launch_pdl(kern, dim3(N / tc::BN, M / tc::BM), dim3(tc::kThreads), tc::smem_bytes(NS), st, a2[0], a2[1],
+                        bh, bl, args);
 }
 
 template <int MODE, bool A_MN, bool B_MN>
@@ -266,9 +273,8 @@ static int pack_weights(dg_mlp *mm) {
 static int forward(dg_mlp *mm, int n) {
   const int Bp = round_up(n, tc::BM);
   const int cnt = Bp * mm->pin[0];
-  k_x_to_split<<<(cnt + 255) / 256 < 1024 ? (cnt + 255) / 256 : 1024, 256, 0, mm->st>>>(n, mm->n_in, mm->pin[0], Bp,
-                                                                                          mm->Xf, mm->Xs);
-  MK2(cudaGetLastError());
+  MK2(dg::launch_pdl(k_x_to_split, dim3((cnt + 255) / 256 < 1024 ? (cnt + 255) / 256 : 1024), dim3(256), 0, mm->st, n,
+                     mm->n_in, mm->pin[0], Bp, mm->Xf, mm->Xs));
   const CUtensorMap *in = mm->mXk;
   for (int l = 0; l < mm->nlayers; ++l) {
     GemmArgs a{};
@@ -299,8 +305,7 @@ static int backward(dg_mlp *mm, int n) {
     a.status = mm->status;
     a.out_f32 = mm->g + mm->woff[l]; a.ldo = fi; a.lim_m = fo; a.lim_n = fi;
     MK2((product<tc::kEpiStoreBounded, true, true>(mm->st, dmn, inmn[0], inmn[1], mm->pout[l], mm->pin[l], Bp, a)));
-    k_colsum<<<fo, 256, 0, mm->st>>>(Bp, mm->pout[l], df, mm->g + mm->boff[l]);
-    MK2(cudaGetLastError());
+    MK2(dg::launch_pdl(k_colsum, dim3(fo), dim3(256), 0, mm->st, Bp, mm->pout[l], df, mm->g + mm->boff[l]));
     if (l > 0) {
       // dZ_{l-1} = (dOut W_l) * SiLU'(Z_{l-1})
       GemmArgs b{};
@@ -332,14 +337,13 @@ static int loss_and_grad(dg_mlp *mm, int n, const float *x, const float *tgt, fl
   if (rc) return rc;
   MK2(cudaMemcpyAsync(mm->Xf, x, sizeof(float) * n * mm->n_in, cudaMemcpyHostToDevice, mm->st));
   MK2(cudaMemcpyAsync(mm->Tt, tgt, sizeof(float) * n * mm->n_out, cudaMemcpyHostToDevice, mm->st));
+  MK2(cudaMemsetAsync(mm->loss, 0, sizeof(float), mm->st));
   rc = forward(mm, n);
   if (rc) return rc;
-  MK2(cudaMemsetAsync(mm->loss, 0, sizeof(float), mm->st));
   const int Bp = round_up(n, tc::BM), Pout = mm->pout[mm->nlayers - 1];
   const int cnt = Bp * Pout;
-  k_mse<<<(cnt + 255) / 256 < 64 ? (cnt + 255) / 256 : 64, 256, 0, mm->st>>>(
-      n, mm->n_out, Pout, Bp, 1.f / (n * mm->n_out), mm->Yf, mm->Tt, mm->dYf, mm->dYs, mm->loss);
-  MK2(cudaGetLastError());
+  MK2(dg::launch_pdl(k_mse, dim3((cnt + 255) / 256 < 64 ? (cnt + 255) / 256 : 64), dim3(256), 0, mm->st, n, mm->n_out,
+                     Pout, Bp, 1.f / (n * mm->n_out), mm->Yf, mm->Tt, mm->dYf, mm->dYs, mm->loss));
   rc = backward(mm, n);
   if (rc) return rc;
   if (loss_out) MK2(cudaMemcpyAsync(loss_out, mm->loss, sizeof(float), cudaMemcpyDeviceToHost, mm->st));
