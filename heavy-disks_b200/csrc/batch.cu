@@ -81,8 +81,10 @@ static int batch_enqueue(dg_batch *b) {
     if (br.size() > 1) {
       MixedGroup *grp = b->groups[gi++];
       for (int s = 0; s < steps && !rc; ++s) rc = mixed_group_enqueue_step(grp, h->st);
+      if (!rc) rc = mixed_group_end_steps(grp, h->st);
     } else {
       for (int s = 0; s < steps && !rc; ++s) rc = h->enqueue_step();
+      if (!rc) rc = h->end_steps();
     }
     if (rc) return b->fail(rc, "dg_batch_advance", h->err.c_str());
     cudaEventRecord(b->events[q], h->st);

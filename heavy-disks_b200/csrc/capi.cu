@@ -186,7 +186,7 @@ int dg_handle::build_khat() {
   MK(dmalloc(&spec, (size_t)Nc * M + (ns + 1) / 2));
   double *tmp = reinterpret_cast<double *>(spec + (size_t)Nc * M);
   cudaError_t e = launch_kernel_samples64(tmp, M, p.Nphi, du, dphi, p.eps, st);
-  const FftDisk<double2> d{{tmp, tmp}, nullptr, spec, nullptr, nullptr, nullptr};
+  const FftDisk<double2> d{{tmp, tmp}, nullptr, spec, nullptr, nullptr, nullptr, nullptr};
   if (e == cudaSuccess) e = launch_phi_fwd<double2>(d, 0, M, M, ft, st);
   if (e == cudaSuccess) e = launch_u_khat(spec, M, Nc, ft, Khat, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
@@ -214,13 +214,13 @@ void dg_handle::release() {
 
 // ---------------------------------------------------------------------------------
 // gravity (FP64): kalnajs.hpp:48-63
-int dg_handle::potential64(const double *dSig, double *dOut) {
+int dg_handle::potential64(const double *dSig, double *dOut, bool step) {
   if (products) {
     const double pref = -p.G * du * dphi / (static_cast<double>(M) * p.Nphi);
     MK(setup::potential(dSig, dR32, pref, dSqrtR, dOut, sg, st));
     return DG_OK;
   }
-  const FftDisk<double2> d{{dSig, dSig}, dR32, W, Khat, dPhiScale, dOut};
+  const FftDisk<double2> d{{dSig, dSig}, dR32, W, Khat, dPhiScale, dOut, step ? ctl : nullptr};
   MK(prof_begin(DG_PROF_GRAV_PHI_FWD));
   MK(launch_phi_fwd<double2>(d, 0, p.Nu, ldW, ft, st));
   MK(prof_end(DG_PROF_GRAV_PHI_FWD));
@@ -241,7 +241,7 @@ int dg_handle::enqueue_step() {
   int fm = kForceNone;
   if (p.selfgrav) {
     MK(prof_begin(DG_PROF_GRAVITY));
-    int rc = potential64(S[c], dPhi);
+    int rc = potential64(S[c], dPhi, true);
     if (rc) return rc;
     MK(prof_end(DG_PROF_GRAVITY));
     fm = kForcePhi;
@@ -251,6 +251,13 @@ int dg_handle::enqueue_step() {
                     st));
   MK(prof_end(DG_PROF_HYDRO));
   cur = o;
+  if (ends_own_steps()) MK(launch_step_finalize(ctl, st));
+  return DG_OK;
+}
+
+// The end of the last enqueued step (the next one's gravity takes care of the others).
+int dg_handle::end_steps() {
+  if (!ends_own_steps()) MK(launch_step_finalize(ctl, st));
   return DG_OK;
 }
 
@@ -359,6 +366,7 @@ int dg_handle::enqueue_step_forces(const double *gRh, const double *gph) {
   }
   const int c = cur, o = cur ^ 1;
   MK(launch_hydro64(S[c], VR[c], VP[c], nullptr, gA, gB, fm, PR[c], S[o], VR[o], VP[o], PR[o], ctl, geom, st));
+  MK(launch_step_finalize(ctl, st));
   cur = o;
   return DG_OK;
 }
@@ -409,6 +417,7 @@ int dg_handle::capture_graph() {
   MK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
   int rc = DG_OK;
   for (int k = 0; k < kGraphSteps && !rc; ++k) rc = enqueue_step();
+  if (!rc) rc = end_steps();
   cudaError_t e = cudaStreamEndCapture(st, &g);
   graph_end_flags = loop_flags();
   set_loop_flags(flags_before);
@@ -435,7 +444,7 @@ int dg_handle::run_chunk(int nsteps) {
     int rc = enqueue_step();
     if (rc) return rc;
   }
-  return DG_OK;
+  return end_steps();
 }
 
 // ---------------------------------------------------------------------------------
@@ -630,6 +639,7 @@ static int step_common(dg_handle *h, double dt, const double *gR, const double *
   if (rc) return rc;
   if (own_gravity) {
     rc = h->enqueue_step();
+    if (!rc) rc = h->end_steps();
   } else {
     rc = h->enqueue_step_forces(gR, gp);
   }
@@ -860,6 +870,7 @@ int dg_step_host(dg_handle *h, double cfl, double *Sig, double *vR, double *vp, 
   if (rc) return rc;
   DG_CK(cudaMemcpyAsync(h->hdt, &h->ctl->dt, sizeof(double), cudaMemcpyDeviceToHost, h->st));
   rc = h->enqueue_step();
+  if (!rc) rc = h->end_steps();
   if (rc) return rc;
   rc = h->download_state(Sig, vR, vp);  // synchronises the stream
   if (rc) return rc;
@@ -888,8 +899,10 @@ int dg_tuning_info(const dg_handle *h, char *buf, int len) {
 
 int dg_kernels_per_step(const dg_handle *h) {
   if (!h) return DG_ERR_INVALID;
-  const int grav = !h->p.selfgrav ? 0 : (h->p.precision == DG_PREC_MIXED ? h->mixed_gravity_kernels() : 3);
-  return grav + (h->p.precision == DG_PREC_MIXED ? h->mixed_hydro_kernels() : 1);
+  // (with self-gravity the step's end rides in the next step's gravity)
+  if (h->p.precision == DG_PREC_MIXED)
+    return (h->p.selfgrav ? h->mixed_gravity_kernels() : 0) + h->mixed_hydro_kernels();
+  return h->p.selfgrav ? 4 : 2;
 }
 
 int dg_profile_read(dg_handle *h, double *ms, long long *count) {

@@ -18,6 +18,7 @@ struct dg_handle;
 std::string mixed_group_key(const dg_handle *h, bool with_fused = true);
 MixedGroup *mixed_group_create(const std::vector<dg_handle *> &disks, std::string *err);
 int mixed_group_enqueue_step(MixedGroup *g, cudaStream_t st);
+int mixed_group_end_steps(MixedGroup *g, cudaStream_t st);
 void mixed_group_destroy(MixedGroup *g);
 
 struct dg_handle {
@@ -89,8 +90,10 @@ struct dg_handle {
   int init(const dg_params &pp);
   int build_khat();
   void release();
-  int potential64(const double *dSig, double *dOut);
+  int potential64(const double *dSig, double *dOut, bool step = false);
   int enqueue_step();
+  int end_steps();
+  bool ends_own_steps() const;
   int enqueue_step_forces(const double *gR, const double *gp);
   int set_ctl_fields(double t, double tlim, double cfl, double dt, double tnext, double dtout, int fixed_dt);
   int read_ctl();

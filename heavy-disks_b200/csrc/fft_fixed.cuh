@@ -217,6 +217,7 @@ __global__ void __launch_bounds__(LB, MINB) k_u_conv_n(const FftDisk<V> d,
   const V *tws = fft_table<true>(sm, gtw, P::ntw, flat, nt), *half = fft_table<true>(sm + P::tab, ghalf, N, flat, nt);
   pdl_wait();
   pdl_trigger();
+  if (d.ctl && blockIdx.x == 0 && flat == nt - 1) finalize_pending(d.ctl);
   __syncthreads();
   for (int mode = blockIdx.x; mode < Nc; mode += gridDim.x) {
     V *x = d.W + (size_t)mode * ldw;

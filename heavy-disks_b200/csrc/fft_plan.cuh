@@ -30,6 +30,7 @@ template <typename V> struct FftDisk {
   const T *kr;         // khat in transform order
   const T *outscale;   // per row
   T *out;              // the potential
+  Ctl *ctl;            // whose due hydro end pass 2 finalises, or NULL
 };
 
 // Tables of one transform length for both directions of a grid.

@@ -36,6 +36,7 @@
 #pragma once
 
 #include "fft_plan.cuh"
+#include "step_ctl.cuh"
 
 namespace dg {
 
@@ -371,6 +372,7 @@ __global__ void __launch_bounds__(kFftMaxThreads, 2) k_u_conv(const FftDisk<V> d
   const int last = pl.ns - 1;
   pdl_wait();
   pdl_trigger();
+  if (d.ctl && blockIdx.x == 0 && flat == nt - 1) finalize_pending(d.ctl);
   if (SMT) __syncthreads();
   if (last == 0) {
     fft_mid_any<V>(pl, k, tx, nx, ldg, sts);

@@ -16,6 +16,7 @@ namespace dg {
 cudaError_t launch_hydro64(const double *Sig, const double *vR, const double *vp, const double *Phi,
                            const double *gR, const double *gp, int force_mode, const double *Pin, double *So,
                            double *vRo, double *vpo, double *Po, Ctl *ctl, const Geom64 &g, cudaStream_t st);
+cudaError_t launch_step_finalize(Ctl *ctl, cudaStream_t st);
 cudaError_t launch_pressure64(const double *Sig, double *P, const Geom64 &g, cudaStream_t st);
 cudaError_t launch_cfl64(const double *Sig, const double *vR, const double *vp, Ctl *ctl, const Geom64 &g,
                          int nmodes, int record, cudaStream_t st);

@@ -61,7 +61,7 @@ __global__ void __launch_bounds__(32 * kMaxWarps64, 3) k_hydro64(
         if (!G2) Po[k] = Pin[k];
         lmax = fmax(lmax, cfl_rate64(g, i, So[k], vRo[k], vpo[k]));
       }
-    finish_launch<0>(ctl, si, lmax, msum, red);
+    finish_launch_deferred<0>(ctl, si, lmax, msum, red);
     return;
   }
 
@@ -204,7 +204,17 @@ __global__ void __launch_bounds__(32 * kMaxWarps64, 3) k_hydro64(
     for (int q = 0; q < 2 * si.nmodes; ++q) msum[q] = 0.0;
   }
   if (bad) lmax = __longlong_as_double(0x7ff8000000000000ll);
-  finish_launch<0>(ctl, si, lmax, msum, red);
+  finish_launch_deferred<0>(ctl, si, lmax, msum, red);
+}
+
+// The end of a hydro launch that no gravity kernel takes care of.
+__global__ void k_step_finalize(Ctl *ctl) {
+  pdl_trigger();  // the next kernel's prologue may start; it waits for this one's completion
+  pdl_wait();     // every CTA of the hydro launch has folded its sums
+  if (threadIdx.x == 0) finalize_pending(ctl);
+}
+cudaError_t launch_step_finalize(Ctl *ctl, cudaStream_t st) {
+  return launch_pdl(k_step_finalize, dim3(1), dim3(32), 0, st, ctl);
 }
 
 // CFL reduction over a state (DiskHydro::timestep, hydro.hpp:48-61); the last CTA stores

@@ -685,7 +685,7 @@ int dg_handle::mixed_init_fft() {
   XK(cudaMemcpy(X.rowfac, f.data(), f.size() * sizeof(float), cudaMemcpyHostToDevice));
   k_tab_kr32<<<grid_for((size_t)Nc * M), 256, 0, st>>>(X.kr32, Khat, X.ft32.posU, ft.posU, Nu, 2 * Nc);
   XK(cudaGetLastError());
-  X.fd = FftDisk<float2>{{X.sig[0], X.sig[1]}, X.rowfac, X.W32, X.kr32, X.rowfac + Nu, X.dPhi};
+  X.fd = FftDisk<float2>{{X.sig[0], X.sig[1]}, X.rowfac, X.W32, X.kr32, X.rowfac + Nu, X.dPhi, ctl};
   return DG_OK;
 }
 
@@ -752,7 +752,8 @@ int dg_handle::mixed_init_products() {
       k_tab_tw<<<64, 256, 0, st>>>(X.twp, A, tc::kUcTwLd);
       k_tab_khm<<<grid_for((size_t)nm * 64 * A), 256, 0, st>>>(X.khm, sg.khat, nm, 64 * A, Nphi, X.fused_phi);
       XK(cudaGetLastError());
-      XK(smem_attrs((const void *)tc::k_uconv, tc::kUcSmem));
+      XK(smem_attrs((const void *)tc::k_uconv<false>, tc::kUcSmem));
+      XK(smem_attrs((const void *)tc::k_uconv<true>, tc::kUcSmem));
     }
     if (X.fused_phi) {
       static_assert(tc::kZtModes >= 1024 / 2 + 1 && tc::kZtModes % 32 == 0, "Zt row layout");
@@ -1317,26 +1318,18 @@ int dg_handle::mixed_download_state(double *Sig, double *vRh, double *vph) {
   return DG_OK;
 }
 
-// End of a tile hydro launch: t, dt, records and diagnostics from the sums its CTAs folded
-// into the control block (step_ctl.cuh finish_launch_deferred).
-__global__ void k_step_finalize(Ctl *ctl) {
-  pdl_trigger();  // the next kernel's prologue may start; it waits for this one's completion
-  pdl_wait();     // every CTA of the hydro launch has folded its sums
-  if (threadIdx.x == 0) finalize_launch(ctl, read_step_info(ctl, true, ctl->pend_active));
-}
-
-// the same for every disk of a group (one block per disk)
+// the due hydro ends of every disk of a group (one block per disk)
 __global__ void k_step_finalize_group(const HydroDisk *__restrict__ disks) {
   pdl_trigger();
   pdl_wait();
   Ctl *ctl = disks[blockIdx.x].ctl;
-  if (threadIdx.x == 0) finalize_launch(ctl, read_step_info(ctl, true, ctl->pend_active));
+  if (threadIdx.x == 0) finalize_pending(ctl);
 }
 
 // the step's finalisation after a tile hydro launch (the warp form finalises in its last CTA)
 static cudaError_t launch_finalize(const MixedState &X, Ctl *ctl, cudaStream_t st) {
   if (X.hydro_kind == MixedState::kHydroWarp) return cudaSuccess;
-  return launch_pdl(k_step_finalize, dim3(1), dim3(32), 0, st, ctl);
+  return launch_step_finalize(ctl, st);
 }
 
 static cudaError_t launch_hydro32(MixedState &X, const float *sig, const float *u, const float *w, const float *Phi,
@@ -1438,8 +1431,8 @@ int dg_handle::mixed_gravity() {
     if (X.fused_u) {
       // F1, F2, I1, I2 in one kernel: four modes per CTA, operands kept on chip
       tc::UconvArgs u{X.twp, X.khm, X.Z.hi, X.Z.lo, Nu, Nphi, &ctl->status,
-                      X.fused_phi ? X.Zt.hi : nullptr, X.fused_phi ? X.Zt.lo : nullptr};
-      XK(launch_pdl(tc::k_uconv, dim3(nm / tc::kUcModes), dim3(tc::kUcThreads), tc::kUcSmem, st, X.mRB[0], X.mRB[1],
+                      X.fused_phi ? X.Zt.hi : nullptr, X.fused_phi ? X.Zt.lo : nullptr, ctl};
+      XK(launch_pdl(ends_own_steps() ? tc::k_uconv<false> : tc::k_uconv<true>, dim3(nm / tc::kUcModes), dim3(tc::kUcThreads), tc::kUcSmem, st, X.mRB[0], X.mRB[1],
                     X.mXin[0], X.mXin[1], X.mRA[0], X.mRA[1], X.mRGA[0], X.mRGA[1], X.mRGB[0], X.mRGB[1], u));
     } else {
       // F1: 64-point DFT over i2 (K = 32 complex), twiddle, -> Tb[(i1, ri)][(m, p2)]
@@ -1447,11 +1440,11 @@ int dg_handle::mixed_gravity() {
       XK((gemm<tc::kEpiTwiddleF1, false, true>(X.mRB[0], X.mRB[1], X.mXin[0], X.mXin[1], 128, nm * A, 64, a, st,
                                                  X.ns[1])));
       // F2: A-point DFT over i1, x khat / M -> Yk[(m, p2)][(p1, ri)]
-      a.out_hi = X.Yk.hi; a.out_lo = X.Yk.lo; a.ldo = 2 * A; a.table = X.KW2;
+      a.out_hi = X.Yk.hi; a.out_lo = X.Yk.lo; a.ldo = 2 * A; a.table = X.KW2; a.ctl = ctl;
       XK((gemm<tc::kEpiSplitScaled, true, false>(X.mTb[0], X.mTb[1], X.mRA[0], X.mRA[1], nm * 64, 2 * A, 2 * A, a,
                                                    st, X.ns[2])));
       // I1: inverse A-point DFT over p1, conjugate twiddle -> Ub[(m, i1)][(p2, ri)]
-      a.out_hi = X.Ub.hi; a.out_lo = X.Ub.lo; a.table = nullptr;
+      a.out_hi = X.Ub.hi; a.out_lo = X.Ub.lo; a.table = nullptr; a.ctl = nullptr;
       XK(gemm<tc::kEpiTwiddleI1>(X.mYk[0], X.mYk[1], X.mRGA[0], X.mRGA[1], nm * 64, 2 * A, 2 * A, a, st, X.ns[3]));
       // I2: inverse 64-point DFT over p2 (the 32 physical i2) -> Z[c][i], or at Nphi = 4096
       // the full Hermitian spectrum X[(m / 64, ri)][(m % 64, i)] of the four-step inverse
@@ -1500,9 +1493,10 @@ int dg_handle::mixed_gravity() {
   XK(gemm<tc::kEpiSplit>(X.mFphi[0], X.mFphi[1], X.mSx[0], X.mSx[1], Nphi, Nu, Nphi, a, st, X.ns[0]));
   XK(prof_end(DG_PROF_GRAV_PHI_FWD));
   // G2: Wt[c][p] = KW[c][p] * X1[c][:] . Cu[p][:]
-  a.out_hi = X.Wt.hi; a.out_lo = X.Wt.lo; a.ldo = 2 * Nu; a.table = X.KW;
+  a.out_hi = X.Wt.hi; a.out_lo = X.Wt.lo; a.ldo = 2 * Nu; a.table = X.KW; a.ctl = ctl;
   XK(prof_begin(DG_PROF_GRAV_U));
   XK(gemm<tc::kEpiSplitScaled>(X.mX1[0], X.mX1[1], X.mCu[0], X.mCu[1], Nphi, 2 * Nu, Nu, a, st, X.ns[1]));
+  a.ctl = nullptr;
   // G3: Z[i][c] = CuT[i][:] . Wt[c][:]
   a.out_hi = X.Z.hi; a.out_lo = X.Z.lo; a.ldo = Nphi; a.table = nullptr;
   XK(gemm<tc::kEpiSplit>(X.mCuT[0], X.mCuT[1], X.mWt[0], X.mWt[1], Nu, Nphi, 2 * Nu, a, st, X.ns[2]));
@@ -1521,9 +1515,13 @@ void dg_handle::set_loop_flags(int f) {
   if (mx) mx->prev_rs = (f & 1) != 0;
 }
 
-// the tile forms end with k_step_finalize
+// Whether a step launches its own finalisation: without self-gravity, and at 1024^2, where the
+// row-tile hand-over hides that kernel (46.4 us a step; 47.1 with the finalisation compiled into
+// k_uconv).
+bool dg_handle::ends_own_steps() const { return !p.selfgrav || (mx && mx->fused_phi); }
+
 int dg_handle::mixed_hydro_kernels() const {
-  return (mx && mx->hydro_kind != MixedState::kHydroWarp) ? 2 : 1;
+  return (mx && mx->hydro_kind != MixedState::kHydroWarp && ends_own_steps()) ? 2 : 1;
 }
 
 int dg_handle::mixed_gravity_kernels() const {
@@ -1556,8 +1554,8 @@ int dg_handle::mixed_enqueue_step() {
   XK(launch_hydro32(X, X.sig[c], X.u[c], X.w[c], X.dPhi, nullptr, nullptr, fm, X.sig[o], X.u[o], X.w[o], ctl, st,
                     rs ? X.rowpend : nullptr, fm == kForcePhi, false));
   X.prev_rs = rs;
-  XK(prof_end(DG_PROF_HYDRO));  // the hydro kernel alone; its finalisation follows
-  XK(launch_finalize(X, ctl, st));
+  XK(prof_end(DG_PROF_HYDRO));
+  if (ends_own_steps()) XK(launch_finalize(X, ctl, st));
   if (rs && X.test_stall >= 0) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     XK(cudaStreamIsCapturing(st, &cs));
@@ -1802,8 +1800,6 @@ static int group_launch(MixedGroup *g, cudaStream_t st, bool prepare) {
   dim3 hgrid((Nphi + tj - 1) / tj, (Nu + kTileI - 1) / kTileI, G);
   e = launch_pdl(hk, hgrid, dim3(kThreads32t), hsm, st, (const HydroDisk *)g->hd, b);
   if (e != cudaSuccess) return L->fail(DG_ERR_CUDA, "batch group: hydro", cudaGetErrorString(e));
-  e = launch_pdl(k_step_finalize_group, dim3(G), dim3(32), 0, st, (const HydroDisk *)g->hd);
-  if (e != cudaSuccess) return L->fail(DG_ERR_CUDA, "batch group: finalisation", cudaGetErrorString(e));
   for (dg_handle *h : g->disks) h->cur ^= 1;
   return DG_OK;
 }
@@ -1875,7 +1871,7 @@ MixedGroup *mixed_group_create(const std::vector<dg_handle *> &disks, std::strin
                                   &h->ctl->status, nullptr});
       tc::UconvDisk u{};
       u.xh = X.mXin[0]; u.xl = X.mXin[1];
-      u.a = tc::UconvArgs{XL.twp, X.khm, X.Z.hi, X.Z.lo, Nu, Nphi, &h->ctl->status, X.Zt.hi, X.Zt.lo};
+      u.a = tc::UconvArgs{XL.twp, X.khm, X.Z.hi, X.Z.lo, Nu, Nphi, &h->ctl->status, X.Zt.hi, X.Zt.lo, h->ctl};
       uc.push_back(u);
       pi.push_back(tc::PhiInvArgs{X.Zt.hi, X.Zt.lo, XL.twphi, X.phiscale, X.dPhi, Nphi, &h->ctl->status, nullptr,
                                   0, 0});
@@ -1887,10 +1883,10 @@ MixedGroup *mixed_group_create(const std::vector<dg_handle *> &disks, std::strin
     a.M = Nphi; a.N = Nu; a.K = Nphi; a.out_hi = X.X1.hi; a.out_lo = X.X1.lo; a.ldo = Nu;
     gd[0][k].hi = X.mSx[0]; gd[0][k].lo = X.mSx[1]; gd[0][k].args = a;
     // G2: per-disk A = X1 -> Wt, x KW
-    a.M = Nphi; a.N = 2 * Nu; a.K = Nu; a.out_hi = X.Wt.hi; a.out_lo = X.Wt.lo; a.ldo = 2 * Nu; a.table = X.KW;
+    a.M = Nphi; a.N = 2 * Nu; a.K = Nu; a.out_hi = X.Wt.hi; a.out_lo = X.Wt.lo; a.ldo = 2 * Nu; a.table = X.KW; a.ctl = h->ctl;
     gd[1][k].hi = X.mX1[0]; gd[1][k].lo = X.mX1[1]; gd[1][k].args = a;
     // G3: per-disk B = Wt -> Z
-    a.M = Nu; a.N = Nphi; a.K = 2 * Nu; a.out_hi = X.Z.hi; a.out_lo = X.Z.lo; a.ldo = Nphi; a.table = nullptr;
+    a.M = Nu; a.N = Nphi; a.K = 2 * Nu; a.out_hi = X.Z.hi; a.out_lo = X.Z.lo; a.ldo = Nphi; a.table = nullptr; a.ctl = nullptr;
     gd[2][k].hi = X.mWt[0]; gd[2][k].lo = X.mWt[1]; gd[2][k].args = a;
     // G4: per-disk A = Z -> dPhi (FP32, scaled by -G du dphi / sqrt(R))
     a.M = Nu; a.N = Nphi; a.K = Nphi; a.out_hi = a.out_lo = nullptr; a.out_f32 = X.dPhi; a.ldo = Nphi;
@@ -1924,3 +1920,9 @@ MixedGroup *mixed_group_create(const std::vector<dg_handle *> &disks, std::strin
 }
 
 int mixed_group_enqueue_step(MixedGroup *g, cudaStream_t st) { return group_launch(g, st, false); }
+
+int mixed_group_end_steps(MixedGroup *g, cudaStream_t st) {
+  const cudaError_t e = launch_pdl(k_step_finalize_group, dim3((unsigned)g->disks.size()), dim3(32), 0, st,
+                                   (const HydroDisk *)g->hd);
+  return e == cudaSuccess ? DG_OK : g->lead->fail(DG_ERR_CUDA, "batch group: finalisation", cudaGetErrorString(e));
+}

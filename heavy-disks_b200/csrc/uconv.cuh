@@ -52,6 +52,7 @@ struct UconvArgs {
   // columns 2m, 2m + 1 (the fused inverse phi transform's input, phiinv.cuh; modes above
   // Nphi / 2 stay zero)
   __nv_bfloat16 *zt_hi, *zt_lo;
+  Ctl *ctl;  // whose due hydro end this kernel finalises (FIN forms)
 };
 
 // byte offset of 16-byte chunk ch of row r in a 128-byte-swizzled tile
@@ -90,6 +91,8 @@ __device__ __forceinline__ void uc_stage_sync() {
   tc_fence_after();
 }
 
+// FIN: one warp of the first CTA finalises the step before (a.ctl)
+template <bool FIN>
 __device__ __forceinline__ void uconv_cta(const CUtensorMap *pRBh, const CUtensorMap *pRBl, const CUtensorMap *pXh, const CUtensorMap *pXl, const CUtensorMap *pRAh, const CUtensorMap *pRAl, const CUtensorMap *pRGAh, const CUtensorMap *pRGAl, const CUtensorMap *pRGBh, const CUtensorMap *pRGBl, const UconvArgs &a) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t *sm = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -165,6 +168,11 @@ __device__ __forceinline__ void uconv_cta(const CUtensorMap *pRBh, const CUtenso
   __syncwarp();
   pdl_wait();  // every thread: Z is read by the kernel after this one's predecessor
   pdl_trigger();
+  // (the first product is still running: this warp would wait for it)
+  if (FIN && blockIdx.x == 0) {
+    if (warp == 7 && lane == 0) finalize_pending(a.ctl);
+    __syncwarp();
+  }
   bool ok = mbar_wait(&bar_mma, 0, a.status);
   tc_fence_after();
 
@@ -393,6 +401,7 @@ __device__ __forceinline__ void uconv_cta(const CUtensorMap *pRBh, const CUtenso
   if (warp == 0) tmem_dealloc(tmem, kUcTmemCols);
 }
 
+template <bool FIN>
 __global__ void __launch_bounds__(kUcThreads, 1)
     k_uconv(const __grid_constant__ CUtensorMap tRBh,
     const __grid_constant__ CUtensorMap tRBl,
@@ -404,7 +413,7 @@ __global__ void __launch_bounds__(kUcThreads, 1)
     const __grid_constant__ CUtensorMap tRGAl,
     const __grid_constant__ CUtensorMap tRGBh,
     const __grid_constant__ CUtensorMap tRGBl, UconvArgs a) {
-  uconv_cta(&tRBh, &tRBl, &tXh, &tXl, &tRAh, &tRAl, &tRGAh, &tRGAl, &tRGBh, &tRGBl, a);
+  uconv_cta<FIN>(&tRBh, &tRBl, &tXh, &tXl, &tRAh, &tRAl, &tRGAh, &tRGAl, &tRGBh, &tRGBl, a);
 }
 
 // The same for a group of disks of one grid (batched sweeps): blockIdx.y is the disk; its
@@ -424,7 +433,7 @@ __global__ void __launch_bounds__(kUcThreads, 1)
     const __grid_constant__ CUtensorMap tRGBh,
     const __grid_constant__ CUtensorMap tRGBl, const UconvDisk *__restrict__ disks) {
   const UconvDisk &d = disks[blockIdx.y];
-  uconv_cta(&tRBh, &tRBl, &d.xh, &d.xl, &tRAh, &tRAl, &tRGAh, &tRGAl, &tRGBh, &tRGBl, d.a);
+  uconv_cta<true>(&tRBh, &tRBl, &d.xh, &d.xl, &tRAh, &tRAl, &tRGAh, &tRGAl, &tRGBh, &tRGBl, d.a);
 }
 
 }  // namespace tc
