@@ -251,17 +251,23 @@ def ncu_traffic(precision, size):
         return {}
 
 
+def fft_gravity(precision, Nu, Nphi):
+    """Whether a disk's gravity runs as FFTs (the library's own rule) rather than tensor-core products."""
+    return precision == "fp64" or (Nu * Nphi > 1024 * 1024 and not os.environ.get("DISKGPU_STAGES"))
+
+
 def gravity_parts(precision, Nu, Nphi):
     """(phase, kernel, bound, work per launch, unit of work) of the three gravity parts."""
-    M = 2 * Nu
-    if precision == "fp64":
-        # HBM-bound FFT passes; algorithmic bytes: Sigma in + half spectrum out (phi forward),
-        # spectrum in/out + khat (u convolution), spectrum in + Phi out (phi inverse)
-        nc = Nphi // 2 + 1
-        spec = 16 * M * nc
-        return [("grav_phi_fwd", "FP64 smem FFT, phi forward (k_phi_fwd)", "hbm", 8 * Nu * Nphi + spec, "B"),
-                ("grav_u", "FP64 smem FFT, u convolution x khat (k_u_conv)", "hbm", 2 * spec + spec, "B"),
-                ("grav_phi_inv", "FP64 smem FFT, phi inverse + scaling (k_phi_inv)", "hbm", spec + 8 * Nu * Nphi, "B")]
+    # FP64, and mixed disks above 2^20 zones in FP32: FFTs in shared memory.  Algorithmic bytes:
+    # Sigma in + half spectrum out (phi forward), spectrum in and out + real khat (u convolution),
+    # spectrum in + Phi out (phi inverse)
+    if fft_gravity(precision, Nu, Nphi):
+        word, name = (8, "FP64") if precision == "fp64" else (4, "FP32")
+        spec, field = 2 * word * Nu * (Nphi // 2 + 1), word * Nu * Nphi
+        khat = word * 2 * Nu * (Nphi // 2 + 1)
+        return [("grav_phi_fwd", name + " shared-memory FFT, phi forward", "hbm", field + spec, "B"),
+                ("grav_u", name + " shared-memory FFT, u convolution x khat", "hbm", 2 * spec + khat, "B"),
+                ("grav_phi_inv", name + " shared-memory FFT, phi inverse + scaling", "hbm", spec + field, "B")]
     # split-BF16 tcgen05 products: 3 MMAs per term, 2 flops per MAC
     g1 = 6 * Nphi * Nu * Nphi
     g1name = "phi DFT GEMM (k_gemm_split, split-BF16)"
@@ -567,9 +573,9 @@ def main():
     hbm_peak, tc_peak, peak_kind = measured_peaks()
     traffic = ncu_traffic(a.precision, N)
     word = 8 if a.precision == "fp64" else 4
-    # read Sigma, vR, vphi, Phi; write Sigma, vR, vphi (+ the split-BF16 gravity operand,
-    # 2 x 2 bytes, that the mixed hydro kernel writes for the next step's gravity)
-    hyd_bytes = (7 * word + (4 if a.precision == "mixed" else 0)) * zones
+    # read Sigma, vR, vphi, Phi; write Sigma, vR, vphi (+ the split-BF16 gravity operand, 2 x 2
+    # bytes, that the mixed hydro kernel writes where the next step's gravity is tensor-core products)
+    hyd_bytes = (7 * word + (0 if fft_gravity(a.precision, N, N) else 4)) * zones
 
     def entry(phase, kernel, bound, work, unit_kind):
         t, n = prof.get(phase, (0.0, 0))

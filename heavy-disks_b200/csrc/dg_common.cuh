@@ -16,7 +16,8 @@ constexpr int kMaxModes = 9;        // C_0 .. C_8 accumulated on device
 constexpr int kMaxRecords = 4096;   // device ring of mode records between host drains
 
 // Device-resident control block of one disk: the step loop runs without host sync.
-// Written only by the last CTA of the hydro kernel (and by host-side set-up).
+// Written by the hydro's CTAs (sums) and the end of their launch (step_ctl.cuh), and by
+// host-side set-up.
 struct Ctl {
   // --- host-written configuration (copied as one prefix, up to dtinv_bits) ---
   double t;          // simulation time at the start of the next step (advanced by the device)

@@ -7,14 +7,14 @@ namespace dg {
 
 // ---------------------------------------------------------------------------------
 // End-of-launch bookkeeping shared by the hydro and CFL kernels.  Every CTA folds its
-// partial max of (sR + sphi) and its mode sums into the control block; the last CTA to
-// finish advances t, derives the next dt (diskmain.cpp:100-101: dt = cfl / max, clipped
-// so that t lands on tlim), appends a mode record when one is due (diskmain.cpp:93-99),
-// and resets the accumulators for the next launch.
+// partial max of (sR + sphi) and its mode sums into the control block; the end of the launch
+// (the last CTA, or later by finalize_pending) advances t, derives the next dt
+// (diskmain.cpp:100-101: dt = cfl / max, clipped so that t lands on tlim), appends a mode
+// record when one is due (diskmain.cpp:93-99), and resets the accumulators.
 struct StepInfo {
   double t, dt, tlim;
   bool active;     // this launch advances the state
-  bool advance_t;  // the last CTA adds dt to t (hydro launches)
+  bool advance_t;  // the end of the launch adds dt to t (hydro launches)
   bool record;     // the new state is due for a mode record
   int nmodes;      // number of m accumulated (0 = none)
 };
