@@ -48,7 +48,7 @@ template <typename V, int N> struct FixedLen {
     cudaError_t e = cudaSuccess;
     for (const void *f : {(const void *)k_phi_fwd_n<V, N, LB, MINB>, (const void *)k_u_conv_n<V, N, LBU, MINBU>,
                           (const void *)k_phi_inv_n<V, N, LB, MINB>}) {
-      if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+      if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem);
       if (e == cudaSuccess)
         e = cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
     }

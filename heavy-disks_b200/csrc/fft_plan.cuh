@@ -8,6 +8,7 @@ namespace dg {
 
 constexpr int kFftMaxStages = 14;   // 2^13 = 8192 by radix 2 alone
 constexpr int kFftMaxThreads = 512;
+constexpr size_t kMaxSmem = 227 * 1024;  // dynamic shared memory of a CTA (sm_100a)
 
 // One length's stage list, kept by the host with its device tables.
 struct FftPlan {

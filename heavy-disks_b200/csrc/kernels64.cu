@@ -537,11 +537,18 @@ cudaError_t build_fft_tables(int Nu, int Nphi, FftTables<V> *ft) {
   return e;
 }
 
+// Lengths whose tables go to shared memory (the SMT forms).
+static bool fft_smt(int n) { return n <= 512; }
+
 // Transforms per CTA: up to 4 (their rows share the 128-byte runs of W), while every SM
-// still gets a CTA.
-static int fft_log2_batch(const FftPlan &pl, int count) {
+// still gets a CTA and they fit its shared memory with their tables (two FP64 transforms do up
+// to some 6300 points; one of 8192 takes 150 KB).
+template <typename V> static int fft_log2_batch(const FftPlan &pl, int count) {
+  const size_t one = fft_pad_len<V>(pl.n), tab = fft_smt(pl.n) ? fft_tab_phi<V>(pl.n, pl.ntw) : 0;
   int lg = 0;
-  while (lg < 2 && (pl.threads << (lg + 1)) <= kFftMaxThreads && ((count) >> (lg + 1)) >= sm_count()) ++lg;
+  while (lg < 2 && (pl.threads << (lg + 1)) <= kFftMaxThreads && (count >> (lg + 1)) >= sm_count() &&
+         ((one << (lg + 1)) + tab) * sizeof(V) <= kMaxSmem)
+    ++lg;
   return lg;
 }
 
@@ -567,15 +574,12 @@ cudaError_t prepare_fft_kernels() {
   return cudaSuccess;
 }
 
-// Lengths whose tables go to shared memory (the SMT forms).
-static bool fft_smt(int n) { return n <= 512; }
-
 template <typename V>
 cudaError_t launch_phi_fwd(const FftDisk<V> &d, int b, int nrows, int ldw,
                            const FftTables<V> &ft, cudaStream_t st) {
   const FftPlan &pl = ft.phi;
   if (pl.fixed && nrows % 2 == 0) return fixed_phi_fwd<V>(pl.n, d, b, nrows, ldw, ft.twPhi, st);
-  const int pairs = (nrows + 1) / 2, lg = fft_log2_batch(pl, pairs), nb = 1 << lg;
+  const int pairs = (nrows + 1) / 2, lg = fft_log2_batch<V>(pl, pairs), nb = 1 << lg;
   const bool smt = fft_smt(pl.n);
   const size_t sm = ((size_t)nb * fft_pad_len<V>(pl.n) + (smt ? fft_tab_phi<V>(pl.n, pl.ntw) : 0)) * sizeof(V);
   return launch_pdl(smt ? k_phi_fwd<V, true> : k_phi_fwd<V, false>, dim3((pairs + nb - 1) / nb),
@@ -598,7 +602,7 @@ cudaError_t launch_phi_inv(const FftDisk<V> &d, int nrows, int ldw,
                            const FftTables<V> &ft, cudaStream_t st) {
   const FftPlan &pl = ft.phi;
   if (pl.fixed && nrows % 2 == 0) return fixed_phi_inv<V>(pl.n, d, nrows, ldw, ft.twPhi, st);
-  const int pairs = (nrows + 1) / 2, lg = fft_log2_batch(pl, pairs), nb = 1 << lg;
+  const int pairs = (nrows + 1) / 2, lg = fft_log2_batch<V>(pl, pairs), nb = 1 << lg;
   const bool smt = fft_smt(pl.n);
   const size_t sm = ((size_t)nb * fft_pad_len<V>(pl.n) + (smt ? fft_tab_phi<V>(pl.n, pl.ntw) : 0)) * sizeof(V);
   return launch_pdl(smt ? k_phi_inv<V, true> : k_phi_inv<V, false>, dim3((pairs + nb - 1) / nb),

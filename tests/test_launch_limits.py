@@ -1,0 +1,94 @@
+"""Launch shapes of the transforms against the shared-memory limits, without a GPU: the
+library's own objects linked with a stand-in for the CUDA runtime (fake_cudart.cpp) that
+refuses what the runtime would refuse.  The child process makes handles through the C ABI and
+asks each for a potential; memory copies and kernels do nothing."""
+import json
+import os
+import subprocess
+import sys
+
+import pytest
+
+from helpers import ROOT
+
+PKG = os.path.join(ROOT, "heavy-disks_b200")
+
+
+@pytest.fixture(scope="module")
+def fake_lib(tmp_path_factory):
+    subprocess.run(["make", "-s", "-C", PKG], check=True)
+    out = str(tmp_path_factory.mktemp("fake") / "libdiskgpu_fake.so")
+    objs = [os.path.join(PKG, "build", f) for f in sorted(os.listdir(os.path.join(PKG, "build"))) if f.endswith(".o")]
+    inc = os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "include")
+    subprocess.run(["g++", "-O1", "-std=c++17", "-shared", "-fPIC", "-I" + inc,
+                    os.path.join(ROOT, "tests", "fake_cudart.cpp"), *objs, "-o", out], check=True)
+    return out
+
+
+CHILD = r"""
+import ctypes as C, json, sys
+sys.path.insert(0, sys.argv[1])
+import diskgpu as D
+D.LIB_PATH = sys.argv[2]
+L = D.lib()
+L.fake_max_smem.restype = C.c_size_t
+bad, smem = [], 0
+host = (C.c_double * 1)()
+for Nu, Nphi, prec, dev in json.loads(sys.argv[3]):
+    L.fake_reset()
+    p = D.default_params(Nu=Nu, Nphi=Nphi, precision=prec, device=dev)
+    h = C.c_void_p()
+    rc = L.dg_create(C.byref(p), C.byref(h))
+    if rc == 0:
+        rc = L.dg_potential(h, host, host)
+        L.dg_destroy(h)
+    smem = max(smem, L.fake_max_smem())
+    if rc or L.fake_refused():
+        bad.append((Nu, Nphi, prec, dev, rc))
+print(json.dumps([bad, smem]))
+"""
+
+
+def refused(lib, grids):
+    r = subprocess.run([sys.executable, "-c", CHILD, PKG, lib, json.dumps(grids)], capture_output=True, text=True,
+                       check=True)
+    return json.loads(r.stdout.splitlines()[-1])
+
+
+def smooth(lo, hi):
+    def ok(n):
+        for p in (2, 3, 5):
+            while n % p == 0:
+                n //= p
+        return n == 1
+    return [n for n in range(lo, hi + 1) if ok(n)]
+
+
+def test_every_accepted_length_launches(fake_lib):
+    """Every length of either direction, beside few, some and many transforms of it."""
+    grids = [(Nu, Nphi, "fp64", 0) for Nphi in smooth(2, 8192) for Nu in (6, 300, 4096)]
+    grids += [(Nu, Nphi, "fp64", 0) for Nu in smooth(2, 4096) for Nphi in (9, 640, 8192)]
+    grids += [(Nu, Nphi, "mixed", 0) for Nphi in smooth(2, 8192) if Nphi % 128 == 0
+              for Nu in (128, 384, 640, 4096)]
+    bad, smem = refused(fake_lib, grids)
+    assert bad == []
+    assert smem > 100 * 1024  # the stand-in saw the large transforms
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("Nu,Nphi,prec", [(300, 8192, "fp64"), (640, 6400, "fp64"), (405, 7500, "fp64"),
+                                          (1000, 6250, "fp64"), (384, 8192, "mixed")])
+def test_potential_of_many_long_rows(Nu, Nphi, prec):
+    """The same on the GPU, values included: the bounds of the other potential tests over
+    lengths, 1e-12 (FP64) and 1e-6 (FP32 transforms)."""
+    import numpy as np
+
+    import diskgpu as D
+    import oracle as O
+    from helpers import rel_err
+    r = np.random.RandomState(Nu * 8209 + Nphi)
+    Sig = r.uniform(0.1, 1.0, (Nu, Nphi))
+    want = O.Kalnajs(Nu, Nphi, eps=0.01).potential(Sig)
+    with D.Disk(Nu, Nphi, eps=0.01, precision=prec) as d:
+        got = d.potential(Sig)
+    assert rel_err(got, want) < (1e-12 if prec == "fp64" else 1e-6)
