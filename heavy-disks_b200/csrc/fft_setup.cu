@@ -42,11 +42,8 @@ static FftShape fft_shape(int n, int count) {
   return s;
 }
 
-
-
+// (for each handle: the limit belongs to the device)
 static cudaError_t prepare_kernels() {
-  static bool done = false;
-  if (done) return cudaSuccess;
   int dev = 0, optin = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
@@ -56,7 +53,6 @@ static cudaError_t prepare_kernels() {
     cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
     if (e != cudaSuccess) return e;
   }
-  done = true;
   return cudaSuccess;
 }
 

@@ -1,6 +1,7 @@
 // Plain-method (FP64) kernels: fused hydro step, CFL reduction, forces, mode sums,
 // Kalnajs kernel samples, and launchers for the shared-memory FFT passes.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 
 #include "kernels.h"
@@ -330,13 +331,12 @@ __global__ void k_conserved64(const double *__restrict__ Sig, const double *__re
 // ---------------------------------------------------------------------------------
 // host launchers
 int sm_count() {
-  static int n = 0;
-  if (!n) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-    if (n <= 0) n = 148;
-  }
+  static std::atomic<int> known[64];  // by device; 0: not asked yet
+  int dev = 0, n = 0;
+  cudaGetDevice(&dev);
+  if (dev >= 0 && dev < 64 && (n = known[dev].load(std::memory_order_relaxed)) > 0) return n;
+  if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
+  if (dev >= 0 && dev < 64) known[dev].store(n, std::memory_order_relaxed);
   return n;
 }
 
@@ -552,10 +552,9 @@ template <typename V> static int fft_log2_batch(const FftPlan &pl, int count) {
   return lg;
 }
 
-// Raise the dynamic shared-memory limit of every FFT pass once, outside any graph capture.
+// Raise the dynamic shared-memory limit of every FFT pass, for each handle: the limit belongs to
+// the device, and a process may have handles on several.
 cudaError_t prepare_fft_kernels() {
-  static bool done = false;
-  if (done) return cudaSuccess;
   int dev = 0, optin = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
@@ -570,7 +569,6 @@ cudaError_t prepare_fft_kernels() {
     cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
     if (e != cudaSuccess) return e;
   }
-  done = true;
   return cudaSuccess;
 }
 

@@ -75,6 +75,17 @@ def test_every_accepted_length_launches(fake_lib):
     assert smem > 100 * 1024  # the stand-in saw the large transforms
 
 
+def test_second_device_of_a_process(fake_lib):
+    """The limits belong to a device: handles on the process's second and third one launch like
+    those on the first (passes of more than 48 KB: u from 1350 points, phi in batches of rows,
+    and the set-up transforms of a mixed disk)."""
+    sizes = [(1350, 64, "fp64"), (4096, 9, "fp64"), (640, 1000, "fp64"), (6, 8192, "fp64"), (1024, 1024, "fp64"),
+             (2048, 128, "mixed"), (256, 4096, "mixed"), (384, 8192, "mixed")]
+    bad, smem = refused(fake_lib, [s + (dev,) for dev in (0, 1, 2) for s in sizes])
+    assert bad == []
+    assert smem > 48 * 1024
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("Nu,Nphi,prec", [(300, 8192, "fp64"), (640, 6400, "fp64"), (405, 7500, "fp64"),
                                           (1000, 6250, "fp64"), (384, 8192, "mixed")])
