@@ -47,12 +47,14 @@ __device__ __forceinline__ float vanleer32(float a, float b) {
 // The new sigma from its old value and the increments of both sweeps in one rounding
 // (Rows32::one_round; dsr = sigma_dr32, the radial increment).  On fine grids the radial
 // increment is a few units in the last place of sigma; rounded by itself it errs alike over
-// long stretches of a row and over many steps, which adds up in the total mass: 300 steps of
-// the 4096^2 seed drift by 1.3e-11 with two roundings and by 1.1e-13 with one.  Disks
-// on FFT gravity of 2^21 zones or more take the one.  Smaller ones have coarser increments,
-// and under the tensor-core gravity the noise of its split-BF16 operands (16 times the FFT's)
-// breaks those stretches up; they keep the two, since in a drained edge (see mixed_fft_grid)
-// the last place of sigma is what is left of the density.
+// long stretches of a row and over many steps, which adds up in the total mass.  Drift of the
+// standard disk's seed over 300 steps, two roundings / one: 1.3e-11 / 1.1e-13 at 4096^2,
+// 5.6e-11 / 8.2e-14 at 1152^2, 5.0e-11 / 6.4e-13 at 1280 x 1024, 4.0e-11 / 3.1e-12 at
+// 1536 x 1280; after 600 steps two reach 1.1e-10, one stays under 5e-12.  Disks on FFT gravity
+// take the one.  Under the tensor-core gravity the noise of its split-BF16 operands (16 times
+// the FFT's) breaks those stretches up (1152^2: 1.3e-12, 1280 x 1024: 3.7e-12); those disks
+// keep the two, since in a drained edge (see mixed_fft_grid) the last place of sigma is what is
+// left of the density.
 __device__ __forceinline__ float sigma_dr32(float dt, float dF, float iv) { return __fmul_rn(__fmul_rn(dt, dF), iv); }
 __device__ __forceinline__ float sigma_new32(float s, float dsr, float dt, float dF, float iv) {
   return __fadd_rn(s, __fmaf_rn(__fmul_rn(dt, dF), iv, dsr));

@@ -1060,7 +1060,7 @@ static int build_basic(dg_handle *h, const double *Sig, const double *vp) {
   g.invdu = (float)(1.0 / h->du); g.inv2du = (float)(1.0 / (2.0 * h->du));
   g.Kpoly = (float)K; g.gamma = (float)gam; g.gmstar = (float)p.gmstar;
   g.gamma2 = (gam == 2.0) ? 1 : 0;
-  g.one_round = (X.fft && (size_t)Nu * Nphi >= (size_t)1 << 21) ? 1 : 0;
+  g.one_round = X.fft ? 1 : 0;
   return DG_OK;
 }
 
