@@ -149,7 +149,7 @@ __global__ void __launch_bounds__(32 * kMaxWarps64, 3) k_hydro64(
           const double *t = tc - 3 * kRow64W;
           const double cv = t[hCvol];
           const double ns = fma(cv, F0 - F, S3);
-          const double mR = fma(cv, FR0 - FR, S3 * u3), mP = fma(cv, FP0 - FP, S3 * w3);
+          const double mR = fma(S3, u3, cv * (FR0 - FR)), mP = fma(S3, w3, cv * (FP0 - FP));
           double d = dmax_ref(ns, 1e-10);
           double y = rcp_approx64(d);
           const double a = quot64(mR, d, y), b = quot64(mP, d, y);
@@ -166,7 +166,7 @@ __global__ void __launch_bounds__(32 * kMaxWarps64, 3) k_hydro64(
           const double bf = fma(h, up ? qBm : qB, up ? bm : b);
           const double G = vf * sf * t[hAphi], GR = G * af, GP = G * bf;
           const double n2 = fma(cv, G - dn1(G), ns);
-          const double mR2 = fma(cv, GR - dn1(GR), ns * a), mP2 = fma(cv, GP - dn1(GP), ns * b);
+          const double mR2 = fma(ns, a, cv * (GR - dn1(GR))), mP2 = fma(ns, b, cv * (GP - dn1(GP)));
           d = dmax_ref(n2, 1e-10);  // the quotients' floor and the state's (hydro.hpp:69)
           y = rcp_approx64(d);
           const double uo = quot64(mR2, d, y), wo = quot64(mP2, d, y);
