@@ -440,27 +440,30 @@ __device__ __forceinline__ void hydro32p_tile(
         const F2 w3 = mul(fma(mul(S(dt), sub(fg, fg1)), S(iv), mul(sn2, w2)), rd);
         s3 = make_float2(flx ? 1e-10f - S0 : s3.x, fly ? 1e-10f - S0 : s3.y);
         const size_t q = (size_t)i * Nphi + jc;
+        __nv_bfloat162 h2, l2;
+        if (SX) {  // split-BF16 operand: one packed conversion per plane, the roundings of split_bf16
+          const F2 xr = mul(S(c2.w), s3);
+          h2 = __floats2bfloat162_rn(xr.x, xr.y);
+          const float2 hf = __bfloat1622float2(h2);
+          l2 = __floats2bfloat162_rn(xr.x - hf.x, xr.y - hf.y);
+        }
         if (outx && outy) {
           *reinterpret_cast<F2 *>(so + q) = s3;
           *reinterpret_cast<F2 *>(uo + q) = u3;
           *reinterpret_cast<F2 *>(wo + q) = w3;
-        } else if (outx) {  // one half of the pair is output (tile edges)
-          so[q] = s3.x; uo[q] = u3.x; wo[q] = w3.x;
-        } else {
-          so[q + 1] = s3.y; uo[q + 1] = u3.y; wo[q + 1] = w3.y;
-        }
-        if (SX) {  // one packed conversion per plane, the roundings of split_bf16
-          const F2 xr = mul(S(c2.w), s3);
-          const __nv_bfloat162 h2 = __floats2bfloat162_rn(xr.x, xr.y);
-          const float2 hf = __bfloat1622float2(h2);
-          const __nv_bfloat162 l2 = __floats2bfloat162_rn(xr.x - hf.x, xr.y - hf.y);
-          if (outx && outy) {
+          if (SX) {
             *reinterpret_cast<__nv_bfloat162 *>(Sx.hi + q) = h2;
             *reinterpret_cast<__nv_bfloat162 *>(Sx.lo + q) = l2;
-          } else if (outx) {
+          }
+        } else if (outx) {  // one half of the pair is output (tile edges)
+          so[q] = s3.x; uo[q] = u3.x; wo[q] = w3.x;
+          if (SX) {
             Sx.hi[q] = h2.x;
             Sx.lo[q] = l2.x;
-          } else {
+          }
+        } else {
+          so[q + 1] = s3.y; uo[q + 1] = u3.y; wo[q + 1] = w3.y;
+          if (SX) {
             Sx.hi[q + 1] = h2.y;
             Sx.lo[q + 1] = l2.y;
           }
