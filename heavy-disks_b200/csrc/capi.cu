@@ -247,8 +247,9 @@ int dg_handle::enqueue_step() {
     fm = kForcePhi;
   }
   MK(prof_begin(DG_PROF_HYDRO));
-  MK(launch_hydro64(S[c], VR[c], VP[c], dPhi, nullptr, nullptr, fm, PR[c], S[o], VR[o], VP[o], PR[o], ctl, geom,
-                    st));
+  MK(launch_hydro64(S[c], VR[c], VP[c], dPhi, nullptr, nullptr, fm, pr_known ? PR[c] : nullptr, S[o], VR[o], VP[o],
+                    PR[o], ctl, geom, st));
+  pr_known = true;
   MK(prof_end(DG_PROF_HYDRO));
   cur = o;
   if (ends_own_steps()) MK(launch_step_finalize(ctl, st));
@@ -338,7 +339,8 @@ int dg_handle::cfl_launch(int nmodes, int record) {
     int rc = mixed_cfl_launch(nmodes, record);
     if (rc) return rc;
   } else {
-    MK(launch_cfl64(S[cur], VR[cur], VP[cur], ctl, geom, nmodes, record, st));
+    MK(launch_cfl64(S[cur], VR[cur], VP[cur], pr_known ? nullptr : PR[cur], ctl, geom, nmodes, record, st));
+    pr_known = true;
   }
   MK(prof_end(DG_PROF_CFL));
   return DG_OK;
@@ -365,7 +367,9 @@ int dg_handle::enqueue_step_forces(const double *gRh, const double *gph) {
     fm = kForceArrays;
   }
   const int c = cur, o = cur ^ 1;
-  MK(launch_hydro64(S[c], VR[c], VP[c], nullptr, gA, gB, fm, PR[c], S[o], VR[o], VP[o], PR[o], ctl, geom, st));
+  MK(launch_hydro64(S[c], VR[c], VP[c], nullptr, gA, gB, fm, pr_known ? PR[c] : nullptr, S[o], VR[o], VP[o], PR[o], ctl,
+                    geom, st));
+  pr_known = true;
   MK(launch_step_finalize(ctl, st));
   cur = o;
   return DG_OK;
@@ -386,10 +390,10 @@ int dg_handle::conserved_launch(double *out2) {
 int dg_handle::upload_state(const double *Sig, const double *vRh, const double *vph) {
   if (p.precision == DG_PREC_MIXED) return mixed_upload_state(Sig, vRh, vph);
   const size_t n = (size_t)p.Nu * p.Nphi;
+  pr_known = false;
   MK(cudaMemcpyAsync(S[cur], Sig, n * sizeof(double), cudaMemcpyHostToDevice, st));
   MK(cudaMemcpyAsync(VR[cur], vRh, n * sizeof(double), cudaMemcpyHostToDevice, st));
   MK(cudaMemcpyAsync(VP[cur], vph, n * sizeof(double), cudaMemcpyHostToDevice, st));
-  if (PR[cur]) MK(launch_pressure64(S[cur], PR[cur], geom, st));
   return DG_OK;
 }
 
@@ -414,13 +418,16 @@ int dg_handle::capture_graph() {
   // enqueue_step keeps host-side flags of what the last enqueued kernels were; recording
   // runs nothing, so they are put back, and a launch of the graph applies their end values
   const int flags_before = loop_flags();
+  const bool known_before = pr_known;
   MK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
+  pr_known = true;  // a launch of the graph follows a CFL pass or a step
   int rc = DG_OK;
   for (int k = 0; k < kGraphSteps && !rc; ++k) rc = enqueue_step();
   if (!rc) rc = end_steps();
   cudaError_t e = cudaStreamEndCapture(st, &g);
   graph_end_flags = loop_flags();
   set_loop_flags(flags_before);
+  pr_known = known_before;
   cur = 0;  // enqueue_step flipped cur kGraphSteps times during capture
   if (rc) { if (g) cudaGraphDestroy(g); return rc; }
   MK(e);
@@ -431,7 +438,7 @@ int dg_handle::capture_graph() {
 }
 
 int dg_handle::run_chunk(int nsteps) {
-  if (nsteps == kGraphSteps && cur == 0 && use_graphs && !prof_on) {
+  if (nsteps == kGraphSteps && cur == 0 && use_graphs && !prof_on && (pr_known || !PR[0])) {
     if (!graph_exec) {
       int rc = capture_graph();
       if (rc) return rc;

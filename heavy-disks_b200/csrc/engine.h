@@ -41,7 +41,11 @@ struct dg_handle {
 
   // plain-method state (ping-pong), forces scratch, gravity workspace
   double *S[2] = {nullptr, nullptr}, *VR[2] = {nullptr, nullptr}, *VP[2] = {nullptr, nullptr};
-  double *PR[2] = {nullptr, nullptr};  // pressure of S[.] (FP64 path, Gamma != 2)
+  // pressure of S[.] (FP64 path, Gamma != 2).  An upload leaves it open (pr_known false): the CFL
+  // pass that starts every run of steps fills it in, and a step taken before that computes the
+  // pressures it needs.
+  double *PR[2] = {nullptr, nullptr};
+  bool pr_known = false;
   int cur = 0;
   double *dPhi = nullptr, *gA = nullptr, *gB = nullptr;
   // phi half spectra [m][i], row stride ldW (Nu rounded up to even), and the real khat table

@@ -32,7 +32,9 @@
 // For Gamma != 2 the pressure is a field of its own: a step computes it once per zone from
 // the density it stores (the CFL rate needs it there anyway) and the next step loads it,
 // instead of a pow per row visit and another per output (768 x 1024, Gamma = 1.75: 95.8 ->
-// 80.1 us a step; 240 x 180: 26.8 -> 21.7).
+// 80.1 us a step; 240 x 180: 26.8 -> 21.7).  An uploaded state has none: the CFL pass before a
+// run of steps stores it beside the rate, and a lone step straight after an upload takes the
+// form with a pow per row visit (a kernel of its own in the upload cost 5 to 8 us there).
 //
 // phi is periodic (wrapped loads).  Rows outside [0, Nu) load the edge row, which is what
 // the reference's clamped pressure and one-sided potential differences read there; slopes

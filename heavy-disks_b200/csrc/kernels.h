@@ -13,12 +13,13 @@
 namespace dg {
 
 // plain-method (FP64) path
+// Pin: the pressure of Sig, or NULL (Gamma = 2, or not known yet); Po takes the new state's
 cudaError_t launch_hydro64(const double *Sig, const double *vR, const double *vp, const double *Phi,
                            const double *gR, const double *gp, int force_mode, const double *Pin, double *So,
                            double *vRo, double *vpo, double *Po, Ctl *ctl, const Geom64 &g, cudaStream_t st);
 cudaError_t launch_step_finalize(Ctl *ctl, cudaStream_t st);
-cudaError_t launch_pressure64(const double *Sig, double *P, const Geom64 &g, cudaStream_t st);
-cudaError_t launch_cfl64(const double *Sig, const double *vR, const double *vp, Ctl *ctl, const Geom64 &g,
+// Po: takes the pressure of Sig, or NULL
+cudaError_t launch_cfl64(const double *Sig, const double *vR, const double *vp, double *Po, Ctl *ctl, const Geom64 &g,
                          int nmodes, int record, cudaStream_t st);
 cudaError_t launch_modes64(const double *Sig, const Geom64 &g, int nmodes, double *out, cudaStream_t st);
 cudaError_t launch_forces64(const double *Phi, double *gR, double *gp, const Geom64 &g, cudaStream_t st);

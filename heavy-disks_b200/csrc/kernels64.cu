@@ -3,6 +3,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cmath>
+#include <type_traits>
 
 #include "kernels.h"
 #include "hydro64.cuh"
@@ -28,8 +29,9 @@ __device__ __forceinline__ double up1(double v) { return __shfl_up_sync(0xffffff
 __device__ __forceinline__ double dn1(double v) { return __shfl_down_sync(0xffffffffu, v, 1); }
 
 // One time step (hydro64.cuh).  blockIdx.x: group of blockDim.x / 32 strips; blockIdx.y: band
-// of `band` rows.
-template <bool G2, int FM>
+// of `band` rows.  PIN: the pressure comes from a field (Gamma != 2, all but the first step of an
+// uploaded state).
+template <bool G2, int FM, bool PIN>
 __global__ void __launch_bounds__(32 * kMaxWarps64, 3) k_hydro64(
     const double *__restrict__ Sig, const double *__restrict__ vR, const double *__restrict__ vp,
     const double *__restrict__ Phi, const double *__restrict__ gRin, const double *__restrict__ gpin,
@@ -59,7 +61,7 @@ __global__ void __launch_bounds__(32 * kMaxWarps64, 3) k_hydro64(
       for (int i = iA; i < iB; ++i) {
         const size_t k = (size_t)i * Nphi + j;
         So[k] = Sig[k]; vRo[k] = vR[k]; vpo[k] = vp[k];
-        if (!G2) Po[k] = Pin[k];
+        if (!G2) Po[k] = PIN ? Pin[k] : pres64(g, Sig[k]);
         lmax = fmax(lmax, cfl_rate64(g, i, So[k], vRo[k], vpo[k]));
       }
     finish_launch_deferred<0>(ctl, si, lmax, msum, red);
@@ -82,7 +84,7 @@ __global__ void __launch_bounds__(32 * kMaxWarps64, 3) k_hydro64(
     int r = iA - 3;
     // the next row, in flight
     int x = at(r);
-    double nS = Sig[x], nU = vR[x], nW = vp[x], nP = G2 ? 0.0 : Pin[x], nPh = FM == kForcePhi ? Phi[x] : 0.0;
+    double nS = Sig[x], nU = vR[x], nW = vp[x], nP = PIN ? Pin[x] : 0.0, nPh = FM == kForcePhi ? Phi[x] : 0.0;
     // row r-1 as loaded; pressure and potential of rows r-1 and r-2
     double S1 = 0, U1 = 0, W1 = 0, P1 = 0, P2 = 0, Ph1 = 0, Ph2 = 0;
     // rows r-2 and r-3 after the source; differences (row r-2) - (row r-3); slopes of row r-3
@@ -92,10 +94,10 @@ __global__ void __launch_bounds__(32 * kMaxWarps64, 3) k_hydro64(
     const double *tc = tab;  // constants of row r
 #pragma unroll 2  // the windows' shifts become renames
     for (int k = 0; r <= iB + 2; ++k, ++r, tc += kRow64W) {
-      const double S = nS, U = nU, W = nW, Ph = nPh, P = G2 ? g.Kpoly * (S * S) : nP;
+      const double S = nS, U = nU, W = nW, Ph = nPh, P = G2 ? g.Kpoly * (S * S) : (PIN ? nP : pres64(g, S));
       x = at(r + 1);
       nS = Sig[x]; nU = vR[x]; nW = vp[x];
-      if (!G2) nP = Pin[x];
+      if (PIN) nP = Pin[x];
       if (FM == kForcePhi) nPh = Phi[x];
       double s1 = 0, u1 = 0, w1 = 0;  // row r-1 after the source
       if (k >= 2) {
@@ -219,10 +221,11 @@ cudaError_t launch_step_finalize(Ctl *ctl, cudaStream_t st) {
 }
 
 // CFL reduction over a state (DiskHydro::timestep, hydro.hpp:48-61); the last CTA stores
-// dt = cfl / max (clipped to tlim unless fixed_dt).  Optionally accumulates mode sums.
+// dt = cfl / max (clipped to tlim unless fixed_dt).  Optionally accumulates mode sums.  Po, if
+// given, takes the pressure, which the rate needs anyway.
 __global__ void __launch_bounds__(256) k_cfl64(const double *__restrict__ Sig, const double *__restrict__ vR,
-                                               const double *__restrict__ vp, Ctl *ctl, Geom64 g, int nmodes,
-                                               int record) {
+                                               const double *__restrict__ vp, double *__restrict__ Po, Ctl *ctl,
+                                               Geom64 g, int nmodes, int record) {
   __shared__ double red[8];
   StepInfo si;
   si.t = ctl->t; si.dt = 0.0; si.tlim = ctl->tlim;
@@ -237,7 +240,14 @@ __global__ void __launch_bounds__(256) k_cfl64(const double *__restrict__ Sig, c
   const size_t n = (size_t)g.Nu * g.Nphi;
   for (size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x) {
     int i = (int)(k / g.Nphi), j = (int)(k % g.Nphi);
-    double r = cfl_rate64(g, i, Sig[k], vR[k], vp[k]);
+    double r;
+    if (Po) {
+      const double s = Sig[k], P = pres64(g, s);
+      Po[k] = P;
+      r = s < 1e-12 ? cfl_rate64(g, i, s, vR[k], vp[k]) : rate64(vR[k], vp[k], cs64(g, s, P), g.invdR[i], g.invdl[i]);
+    } else {
+      r = cfl_rate64(g, i, Sig[k], vR[k], vp[k]);
+    }
     if (!(r == r)) lmax = r;
     else if (lmax == lmax) lmax = fmax(lmax, r);
     if (nmodes) {
@@ -362,34 +372,23 @@ cudaError_t launch_hydro64(const double *Sig, const double *vR, const double *vp
     return launch_pdl(kern, dim3(cols, (g.Nu + band - 1) / band), dim3(32 * wc), 0, st, Sig, vR, vp, Phi, gR, gp, Pin,
                       So, vRo, vpo, Po, ctl, g, band);
   };
-  if (force_mode == kForcePhi) return g.gamma2 ? go(k_hydro64<true, kForcePhi>) : go(k_hydro64<false, kForcePhi>);
-  if (force_mode == kForceArrays)
-    return g.gamma2 ? go(k_hydro64<true, kForceArrays>) : go(k_hydro64<false, kForceArrays>);
-  return g.gamma2 ? go(k_hydro64<true, kForceNone>) : go(k_hydro64<false, kForceNone>);
+  auto pick = [&](auto fm) {
+    constexpr int FM = decltype(fm)::value;
+    if (g.gamma2) return go(k_hydro64<true, FM, false>);
+    return Pin ? go(k_hydro64<false, FM, true>) : go(k_hydro64<false, FM, false>);
+  };
+  if (force_mode == kForcePhi) return pick(std::integral_constant<int, kForcePhi>{});
+  if (force_mode == kForceArrays) return pick(std::integral_constant<int, kForceArrays>{});
+  return pick(std::integral_constant<int, kForceNone>{});
 }
 
-// the pressure field of a state (Gamma != 2)
-__global__ void k_pressure64(const double *__restrict__ Sig, double *__restrict__ P, Geom64 g) {
-  const size_t n = (size_t)g.Nu * g.Nphi;
-  for (size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x)
-    P[k] = pres64(g, Sig[k]);
-}
-
-cudaError_t launch_pressure64(const double *Sig, double *P, const Geom64 &g, cudaStream_t st) {
-  const size_t n = (size_t)g.Nu * g.Nphi;
-  int blocks = (int)((n + 255) / 256);
-  if (blocks > sm_count() * 8) blocks = sm_count() * 8;
-  k_pressure64<<<blocks, 256, 0, st>>>(Sig, P, g);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_cfl64(const double *Sig, const double *vR, const double *vp, Ctl *ctl, const Geom64 &g,
+cudaError_t launch_cfl64(const double *Sig, const double *vR, const double *vp, double *Po, Ctl *ctl, const Geom64 &g,
                          int nmodes, int record, cudaStream_t st) {
   size_t n = (size_t)g.Nu * g.Nphi;
   int blocks = (int)((n + 255) / 256);
   int cap = sm_count() * 4;
   if (blocks > cap) blocks = cap;
-  k_cfl64<<<blocks, 256, 0, st>>>(Sig, vR, vp, ctl, g, nmodes, record);
+  k_cfl64<<<blocks, 256, 0, st>>>(Sig, vR, vp, Po, ctl, g, nmodes, record);
   return cudaGetLastError();
 }
 
