@@ -19,6 +19,7 @@
 #include <map>
 #include <mutex>
 #include <string>
+#include <tuple>
 #include <type_traits>
 #include <utility>
 #include <vector>
@@ -1111,18 +1112,15 @@ int dg_handle::mixed_upload_state(const double *Sig, const double *vRh, const do
 //     records are untouched.  Timed alone the packed and tiled forms differ by less than the
 //     noise, and on some grids the tiled one was picked and cost 2 to 4 us of a 22 us step.
 // A variant must beat the current choice by 2 % to replace it.  Choices are cached per
-// process by (Nu, Nphi, Gamma = 2, self-gravity), so the disks of a batch that share a grid
-// are tuned once.  DISKGPU_TUNE=0 keeps the defaults (packed hydro, stages by K);
-// DISKGPU_HYDRO32 fixes the hydro form; DISKGPU_STAGES asks for the tensor-core products with
-// the given depths.
+// process by (Nu, Nphi, Gamma = 2, self-gravity, form of the gravity), so the disks of a batch
+// that share a grid are tuned once.  DISKGPU_TUNE=0 keeps the defaults (packed hydro, stages by
+// K); DISKGPU_HYDRO32 fixes the hydro form; DISKGPU_STAGES asks for the tensor-core products
+// with the given depths.
 namespace {
 struct TuneKey {
-  int Nu, Nphi, g2, sg;
+  int Nu, Nphi, g2, sg, fft;
   bool operator<(const TuneKey &o) const {
-    if (Nu != o.Nu) return Nu < o.Nu;
-    if (Nphi != o.Nphi) return Nphi < o.Nphi;
-    if (g2 != o.g2) return g2 < o.g2;
-    return sg < o.sg;
+    return std::tie(Nu, Nphi, g2, sg, fft) < std::tie(o.Nu, o.Nphi, o.g2, o.sg, o.fft);
   }
 };
 struct TuneVal {
@@ -1161,7 +1159,7 @@ int dg_handle::mixed_autotune() {
     }
     stages_fixed = true;
   }
-  const TuneKey key{p.Nu, p.Nphi, X.rows.gamma2, p.selfgrav};
+  const TuneKey key{p.Nu, p.Nphi, X.rows.gamma2, p.selfgrav, X.fft};
   {
     std::lock_guard<std::mutex> lk(g_tune_mu);
     auto it = g_tune_cache.find(key);
