@@ -81,7 +81,7 @@ int dg_handle::init(const dg_params &pp) {
     R[i] = std::exp(umin + (i + 0.5) * du);
     Vol[i] = R[i] * (Rf[i + 1] - Rf[i]) * dphi;
     sqrtR[i] = std::sqrt(R[i]);
-    R32[i] = R[i] * sqrtR[i];
+    R32[i] = p.precision == DG_PREC_FP64 ? (double)((long double)R[i] * sqrtl((long double)R[i])) : R[i] * sqrtR[i];
   }
   M = 2 * Nu;
   Nc = Nphi / 2 + 1;
@@ -92,10 +92,15 @@ int dg_handle::init(const dg_params &pp) {
   MK(cudaMemcpy(dRf, Rf.data(), (Nu + 1) * sizeof(double), cudaMemcpyHostToDevice));
   MK(cudaMemcpy(dVol, Vol.data(), Nu * sizeof(double), cudaMemcpyHostToDevice));
   {
-    // the inverse transforms' normalisation and the potential's factor (kalnajs.hpp:58-62)
+    // the inverse transforms' normalisation and the potential's factor (kalnajs.hpp:58-62).  A
+    // row factor's rounding is the same in every step, so errors of its own add up over a run:
+    // the FP64 path's are rounded once, from long double.  (A mixed disk has this gravity for its
+    // basic state alone, and keeps the bits of its FP32 row constants.)
+    const bool once = p.precision == DG_PREC_FP64;
+    const long double prefl = -(long double)p.G * du * dphi / ((long double)M * Nphi);
     const double pref = -p.G * du * dphi / (static_cast<double>(M) * Nphi);
     std::vector<double> ps(Nu);
-    for (int i = 0; i < Nu; ++i) ps[i] = pref / sqrtR[i];
+    for (int i = 0; i < Nu; ++i) ps[i] = once ? (double)(prefl / sqrtl((long double)R[i])) : pref / sqrtR[i];
     MK(cudaMemcpy(dPhiScale, ps.data(), Nu * sizeof(double), cudaMemcpyHostToDevice));
     MK(cudaMemcpy(dSqrtR, sqrtR.data(), Nu * sizeof(double), cudaMemcpyHostToDevice));
   }

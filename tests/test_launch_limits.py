@@ -2,39 +2,18 @@
 library's own objects linked with a stand-in for the CUDA runtime (fake_cudart.cpp) that
 refuses what the runtime would refuse.  The child process makes handles through the C ABI and
 asks each for a potential; memory copies and kernels do nothing."""
-import json
-import os
-import subprocess
-import sys
-
 import pytest
 
-from helpers import ROOT
-
-PKG = os.path.join(ROOT, "heavy-disks_b200")
-
-
-@pytest.fixture(scope="module")
-def fake_lib(tmp_path_factory):
-    subprocess.run(["make", "-s", "-C", PKG], check=True)
-    out = str(tmp_path_factory.mktemp("fake") / "libdiskgpu_fake.so")
-    objs = [os.path.join(PKG, "build", f) for f in sorted(os.listdir(os.path.join(PKG, "build"))) if f.endswith(".o")]
-    inc = os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "include")
-    subprocess.run(["g++", "-O1", "-std=c++17", "-shared", "-fPIC", "-I" + inc,
-                    os.path.join(ROOT, "tests", "fake_cudart.cpp"), *objs, "-o", out], check=True)
-    return out
+from fake_lib import fake_child, fake_lib  # noqa: F401 (a fixture)
 
 
 CHILD = r"""
-import ctypes as C, json, sys
-sys.path.insert(0, sys.argv[1])
-import diskgpu as D
-D.LIB_PATH = sys.argv[2]
+import ctypes as C, json
 L = D.lib()
 L.fake_max_smem.restype = C.c_size_t
 bad, smem = [], 0
 host = (C.c_double * 1)()
-for Nu, Nphi, prec, dev in json.loads(sys.argv[3]):
+for Nu, Nphi, prec, dev in json.loads(arg):
     L.fake_reset()
     p = D.default_params(Nu=Nu, Nphi=Nphi, precision=prec, device=dev)
     h = C.c_void_p()
@@ -50,9 +29,7 @@ print(json.dumps([bad, smem]))
 
 
 def refused(lib, grids):
-    r = subprocess.run([sys.executable, "-c", CHILD, PKG, lib, json.dumps(grids)], capture_output=True, text=True,
-                       check=True)
-    return json.loads(r.stdout.splitlines()[-1])
+    return fake_child(lib, CHILD, grids)
 
 
 def smooth(lo, hi):

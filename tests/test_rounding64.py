@@ -9,6 +9,7 @@ import numpy as np
 import pytest
 
 import diskgpu as D
+from fake_lib import fake_child, fake_lib  # noqa: F401 (a fixture)
 
 LD = np.longdouble
 
@@ -74,3 +75,38 @@ def test_step_rounds_no_more_than_the_scheme_needs(Nu, Nphi, gamma):
     for g, o, e in zip(got, once, want):
         rms = [float(np.sqrt(np.mean((x.astype(LD) - e) ** 2))) for x in (g, o)]
         assert rms[0] <= 1.02 * rms[1], rms
+
+
+CHILD = r"""
+import ctypes as C, json
+import numpy as np
+L = D.lib()
+L.fake_copy.restype = C.POINTER(C.c_double)
+Nu, Nphi, G = json.loads(arg)
+p = D.default_params(Nu=Nu, Nphi=Nphi, G=G)
+h = C.c_void_p()
+assert L.dg_create(C.byref(p), C.byref(h)) == 0
+R, Rf, Vol = np.empty(Nu), np.empty(Nu + 1), np.empty(Nu)
+L.dg_grid(h, D._dp(R), D._dp(Rf), D._dp(Vol))
+n, copies = C.c_longlong(), []
+for k in range(L.fake_copies()):
+    q = L.fake_copy(k, C.byref(n))
+    if n.value == Nu:
+        copies.append(np.ctypeslib.as_array(q, (Nu,)).astype(np.longdouble))
+LD, du, dphi = np.longdouble, (np.log(1.0) - np.log(0.25)) / Nu, 2.0 * np.pi / Nphi
+r = R.astype(LD)
+worst = []
+for want in (r * np.sqrt(r), -LD(G) * LD(du) * LD(dphi) / (LD(2 * Nu) * LD(Nphi)) / np.sqrt(r)):
+    ulp = np.spacing(abs(want).astype(np.float64)).astype(LD)
+    worst.append(min(float(np.max(abs(c - want) / ulp)) for c in copies))
+print(json.dumps(worst))
+"""
+
+
+@pytest.mark.parametrize("Nu,Nphi,G", [(512, 512, 1.0), (240, 180, 1.0), (300, 64, 0.7)])
+def test_row_factors_of_the_gravity_are_rounded_once(fake_lib, Nu, Nphi, G):
+    """What a row is multiplied by before and after the transforms, R^{3/2} and
+    -G du dphi / (M Nphi sqrt(R)), errs alike in every step.  Each is the nearest double to the
+    80-bit value (half a unit in the last place, and what 80 bits leave of it)."""
+    for w in fake_child(fake_lib, CHILD, [Nu, Nphi, G]):
+        assert w <= 0.5 + 2.0 ** -9
