@@ -17,7 +17,7 @@ constexpr size_t kDefaultSmem = 48 * 1024, kOptinSmem = 227 * 1024;
 int g_dev = 0;
 cudaError_t g_last = cudaSuccess;
 std::map<std::pair<int, const void *>, size_t> g_limit;
-long long g_launches = 0, g_refused = 0;
+long long g_launches = 0, g_refused = 0, g_fail_at = -1;
 size_t g_next = 1 << 20, g_max_smem = 0;
 std::vector<std::vector<double>> g_copies;  // small synchronous uploads, in order
 struct Config { dim3 grid, block; size_t smem; cudaStream_t st; } g_cfg;
@@ -30,7 +30,7 @@ cudaError_t launch(const void *f, dim3 g, dim3 b, size_t smem) {
   const auto it = g_limit.find({g_dev, f});
   const size_t lim = it == g_limit.end() ? kDefaultSmem : it->second;
   const bool ok = smem <= lim && g.x && g.y && g.z && b.x && b.x * b.y * b.z <= 1024;
-  ++g_launches;
+  if (g_launches++ == g_fail_at) return done(cudaErrorLaunchOutOfResources);
   if (smem > g_max_smem) g_max_smem = smem;
   if (!ok) ++g_refused;
   return done(ok ? cudaSuccess : cudaErrorInvalidValue);
@@ -40,6 +40,7 @@ cudaError_t launch(const void *f, dim3 g, dim3 b, size_t smem) {
 extern "C" {
 
 // what the test reads
+void fake_fail_at(long long n) { g_fail_at = n; g_launches = 0; }  // launch n from now on fails, -1: none
 long long fake_launches() { return g_launches; }
 long long fake_refused() { return g_refused; }
 size_t fake_max_smem() { return g_max_smem; }

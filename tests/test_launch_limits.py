@@ -63,6 +63,40 @@ def test_second_device_of_a_process(fake_lib):
     assert smem > 48 * 1024
 
 
+FAILS = r"""
+import ctypes as C, json
+L = D.lib()
+host = (C.c_double * 1)()
+out = []
+for Nu, Nphi, prec in json.loads(arg):
+    p = D.default_params(Nu=Nu, Nphi=Nphi, precision=prec)
+    def go():
+        h = C.c_void_p()
+        rc = L.dg_create(C.byref(p), C.byref(h))
+        if rc == 0:
+            rc = L.dg_potential(h, host, host)
+            L.dg_destroy(h)
+        return rc
+    L.fake_fail_at(C.c_longlong(-1))
+    ok = go()
+    n = L.fake_launches()
+    for k in range(n):
+        L.fake_fail_at(C.c_longlong(k))
+        bad = go()
+        L.fake_fail_at(C.c_longlong(-1))
+        out.append((Nu, Nphi, prec, k, ok, bad, go()))
+print(json.dumps(out))
+"""
+
+
+def test_a_failed_launch_is_reported_once(fake_lib):
+    """A launch that the runtime refuses fails the call that made it and no later one."""
+    rows = fake_child(fake_lib, FAILS, [(128, 128, "fp64"), (60, 90, "fp64"), (1152, 1152, "mixed")])
+    assert len(rows) > 18
+    for *what, ok, bad, after in rows:
+        assert ok == 0 and bad == -2 and after == 0, (what, ok, bad, after)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("Nu,Nphi,prec", [(300, 8192, "fp64"), (640, 6400, "fp64"), (405, 7500, "fp64"),
                                           (1000, 6250, "fp64"), (384, 8192, "mixed")])
