@@ -1,6 +1,8 @@
 // The three passes of the Kalnajs convolution (fft_smem.cuh) for lengths known at compile
-// time: 128 .. 4096 as 2^k or 3 2^k, the grids in use.  Same transforms, same tables layout
-// per plan; what the compiler knows here is every stride.
+// time, those of the grids in use: FP64 64, 128, 256, 384, 512, 768, 1024 and 2048
+// (fft_fixed_f64.cu), FP32 256 .. 4096 as 2^k, and 3 2^k and 5 2^k with k >= 7 (fft_fixed_f32.cu).
+// A length is 200 to 270 KB of object code, so every other one takes the runtime form.  Same
+// transforms, same tables layout per plan; what the compiler knows here is every stride.
 //
 // The runtime-length form is bound by instruction issue, two thirds of them index arithmetic
 // (pass 2 at 1024 points, FP32: some 300 instructions per element, issue slots 64 % busy).

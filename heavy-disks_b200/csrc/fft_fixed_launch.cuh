@@ -31,7 +31,8 @@ template <typename V, int N> struct FixedLen {
   static constexpr int LB = 256, MINB = kLong ? 4 : 2, kRegs = 65536 / (LB * MINB);
   static constexpr int LBU = kLong ? 512 : 256, MINBU = kLong ? 1 : 2, kRegsU = 65536 / (LBU * MINBU);
   static constexpr int Q = N / P::LAST;
-  // rows per group: up to 4 pairs (runs of W), while every SM gets a CTA and the rows divide
+  // rows per group: up to 8 pairs (runs of W), to fill a warp or while every SM gets a CTA, and
+  // where the rows divide
   static int log2_batch(int pairs) {
     int lg = 0;
     while (lg < 3 && (Q << (lg + 1)) <= LB && pairs % (2 << lg) == 0 &&

@@ -31,8 +31,9 @@
 // dependence wait, while the previous kernel still runs; long ones leave the tables to L1
 // and the shared memory to more CTAs per SM.  The FP64 pipe's share is the butterflies,
 // about 5 N log2 N operations per transform.  Against out-of-place radix-4 stages with two
-// barriers each and a padded transform in u, 256 FP64 steps: 48.5 -> 37.3 ms at 1024^2,
-// 9.0 -> 7.3 ms at 256^2.
+// barriers each and a padded transform in u, FP64, us a pass (forward / u / inverse, with their
+// launches): 1000^2 21.2 / 43.4 / 20.8 -> 15.0 / 27.5 / 14.6, 640^2 15.1 / 27.1 / 14.7 ->
+// 13.0 / 16.7 / 12.6, 300^2 11.0 / 18.8 / 10.6 -> 9.6 / 12.6 / 10.5.
 #pragma once
 
 #include "fft_plan.cuh"

@@ -113,7 +113,8 @@ struct MixedState {
   FftTables<float2> ft32;
   FftDisk<float2> fd{};
   // Nphi = 4096 on grids whose u convolution runs as four passes: both phi transforms in
-  // two split-BF16 passes each (64 x 64, four-step) instead of the dense DFT products
+  // two split-BF16 passes each (64 x 64, four-step) instead of the dense DFT products.  Such grids
+  // run FFTs by default: this form is for comparisons (DISKGPU_STAGES)
   bool phi4096 = false;
   SplitBuf PhA1, PhB2f, PhB1i, PhB2i, PhT, PhX, PhV;
   float2 *twph = nullptr;  // W_4096^{m1 j2}, [64][64]
