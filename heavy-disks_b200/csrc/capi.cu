@@ -163,7 +163,6 @@ int dg_handle::init(const dg_params &pp) {
   geom.Nu = Nu; geom.Nphi = Nphi; geom.dphi = dphi; geom.du = du;
   geom.Kpoly = p.Kpoly; geom.gamma = p.gamma_gas; geom.gmstar = p.gmstar;
   geom.gamma2 = (p.gamma_gas == 2.0) ? 1 : 0;
-  MK(prepare_fft_kernels());
   int rc = build_khat();
   if (rc) return rc;
   if (p.precision == DG_PREC_MIXED) {

@@ -74,4 +74,14 @@ __device__ __forceinline__ float cfl_rate32(const Rows32 &g, int i, float sig, f
   return (fabsf(u) + cs) * g.invdR[i] + (fabsf(g.V0[i] + w) + cs) * g.invdl[i];
 }
 
+struct SplitBf16 {
+  __nv_bfloat16 *hi, *lo;
+};
+
+__device__ __forceinline__ int wrap_col(int j, int N) {
+  j += (j < 0) ? N : 0;
+  j -= (j >= N) ? N : 0;
+  return j;
+}
+
 }  // namespace dg

@@ -18,7 +18,6 @@
 #pragma once
 
 #include "hydro32.cuh"
-#include "hydro32w.cuh"
 #include "step_ctl.cuh"
 
 namespace dg {

@@ -22,16 +22,6 @@ constexpr int kBand32 = 16;        // radial rows per warp
 constexpr int kOutCols32 = 28;     // output columns per warp
 constexpr int kWarps32 = 4;        // warps per CTA (adjacent strips of one band)
 
-struct SplitBf16 {
-  __nv_bfloat16 *hi, *lo;
-};
-
-__device__ __forceinline__ int wrap_col(int j, int N) {
-  j += (j < 0) ? N : 0;
-  j -= (j >= N) ? N : 0;
-  return j;
-}
-
 __global__ void __launch_bounds__(kWarps32 * 32) k_hydro32w(
     const float *__restrict__ sig, const float *__restrict__ uu, const float *__restrict__ ww,
     const float *__restrict__ Phi, const double *__restrict__ gRin, const double *__restrict__ gpin, int force_mode,

@@ -101,7 +101,6 @@ template <typename V> bool make_fft_plan(int n, FftPlan *pl);
 template <> bool make_fft_plan<double2>(int n, FftPlan *pl);
 template <> bool make_fft_plan<float2>(int n, FftPlan *pl);
 template <typename V> cudaError_t build_fft_tables(int Nu, int Nphi, FftTables<V> *ft);
-cudaError_t prepare_fft_kernels();
 template <typename V>
 cudaError_t launch_phi_fwd(const FftDisk<V> &d, int b, int nrows, int ldw,
                            const FftTables<V> &ft, cudaStream_t st);

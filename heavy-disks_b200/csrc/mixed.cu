@@ -32,7 +32,7 @@
 #include "step_ctl.cuh"
 #include "hydro32w.cuh"
 #include "hydro32t.cuh"
-#include "hydro32p.cuh"
+#include "hydro32p_launch.cuh"
 #include "uconv.cuh"
 #include "phifwd.cuh"
 #include "phiinv.cuh"
@@ -154,23 +154,16 @@ static cudaError_t smem_attrs(const void *fn, size_t bytes) {
   return cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
 }
 
-// every instantiation of the tiled hydro kernels takes more than 48 KB of shared memory
-static cudaError_t hydro32t_prepare() {
+// every instantiation of the tiled hydro kernels takes more than 48 KB of shared memory; sx: of
+// the packed ones, those that write the products' operand or those that do not
+static cudaError_t hydro32t_prepare(bool sx) {
   const void *tile[] = {(const void *)k_hydro32t<true, kForcePhi>, (const void *)k_hydro32t<false, kForcePhi>,
                         (const void *)k_hydro32t<true, kForceArrays>, (const void *)k_hydro32t<false, kForceArrays>,
                         (const void *)k_hydro32t<true, kForceNone>, (const void *)k_hydro32t<false, kForceNone>};
-  const void *packed[] = {
-      (const void *)k_hydro32p<true, kForcePhi, true>,     (const void *)k_hydro32p<false, kForcePhi, true>,
-      (const void *)k_hydro32p<true, kForceArrays, true>,  (const void *)k_hydro32p<false, kForceArrays, true>,
-      (const void *)k_hydro32p<true, kForceNone, true>,    (const void *)k_hydro32p<false, kForceNone, true>,
-      (const void *)k_hydro32p<true, kForcePhi, false>,    (const void *)k_hydro32p<false, kForcePhi, false>,
-      (const void *)k_hydro32p<true, kForceArrays, false>, (const void *)k_hydro32p<false, kForceArrays, false>,
-      (const void *)k_hydro32p<true, kForceNone, false>,   (const void *)k_hydro32p<false, kForceNone, false>};
   cudaError_t e = cudaSuccess;
   for (const void *f : tile)
     if (e == cudaSuccess) e = smem_attrs(f, kSmem32t);
-  for (const void *f : packed)
-    if (e == cudaSuccess) e = smem_attrs(f, kSmem32p);
+  if (e == cudaSuccess) e = sx ? prepare_hydro32p<true>() : prepare_hydro32p<false>();
   return e;
 }
 
@@ -894,7 +887,7 @@ int dg_handle::mixed_init() {
     if (hk && strcmp(hk, "tile") == 0) X.hydro_kind = MixedState::kHydroTile;
     if (Nphi < kLd32t || Nphi % 2) X.hydro_kind = MixedState::kHydroWarp;
     if (X.hydro_kind != MixedState::kHydroWarp) {
-      XK(hydro32t_prepare());
+      XK(hydro32t_prepare(!X.fft));
       bool okh = make_map_f32(&X.mPhi, X.dPhi, Nu, Nphi);
       for (int b = 0; b < 2; ++b)
         okh = okh && make_map_f32(&X.mSig[b], X.sig[b], Nu, Nphi) && make_map_f32(&X.mU[b], X.u[b], Nu, Nphi) &&
@@ -1337,23 +1330,10 @@ static cudaError_t launch_hydro32(MixedState &X, const float *sig, const float *
                                   const double *gR, const double *gp, int fm, float *so, float *uo, float *wo, Ctl *ctl,
                                   cudaStream_t st, int *rowpend, bool early_state, bool finalize) {
   if (X.hydro_kind == MixedState::kHydroPacked) {
-    dim3 grid((X.Nphi + kTileJp - 1) / kTileJp, (X.Nu + kTileI - 1) / kTileI);
-    const SplitBf16 sx{X.Sx.hi, X.Sx.lo};
-    cudaError_t e = cudaSuccess;
     const int b = (sig == X.sig[1]) ? 1 : 0;  // which ping-pong buffer holds the input
-    auto go = [&](auto kern) {
-      e = launch_pdl(kern, grid, dim3(kThreads32t), kSmem32p, st, X.mSig[b], X.mU[b], X.mW[b], X.mPhi, sig, u, w, Phi,
-                     gR, gp, so, uo, wo, sx, ctl, X.rows, rowpend, early_state ? 1 : 0);
-    };
-    const bool g2 = X.rows.gamma2 != 0;
-    auto pick = [&](auto sxc) {
-      constexpr bool SX = decltype(sxc)::value;
-      if (fm == kForcePhi) g2 ? go(k_hydro32p<true, kForcePhi, SX>) : go(k_hydro32p<false, kForcePhi, SX>);
-      else if (fm == kForceArrays) g2 ? go(k_hydro32p<true, kForceArrays, SX>) : go(k_hydro32p<false, kForceArrays, SX>);
-      else g2 ? go(k_hydro32p<true, kForceNone, SX>) : go(k_hydro32p<false, kForceNone, SX>);
-    };
-    if (sx.hi) pick(std::true_type{});
-    else pick(std::false_type{});
+    const Hydro32pArgs a{&X.mSig[b], &X.mU[b], &X.mW[b], &X.mPhi, sig, u, w, Phi, gR, gp, so, uo, wo,
+                         SplitBf16{X.Sx.hi, X.Sx.lo}, ctl, &X.rows, rowpend, early_state ? 1 : 0};
+    cudaError_t e = a.Sx.hi ? launch_hydro32p<true>(a, fm, st) : launch_hydro32p<false>(a, fm, st);
     if (e == cudaSuccess && finalize) e = launch_finalize(X, ctl, st);
     return e;
   }

@@ -78,7 +78,7 @@ struct GemmArgs {
   // sets rowpend[0 .. rp_n) = rp_val once this kernel's predecessor has completed
   int *rowpend;
   int rp_n, rp_val;
-  Ctl *ctl;            // whose due hydro end this product finalises beside its main loop, or NULL
+  Ctl *ctl;            // kEpiSplitScaled: whose due hydro end this product finalises beside its main loop, or NULL
   // surrogate network epilogues
   const float *bias;   // kEpiMlpAct, kEpiMlpOut: per column, padded with zeros
   int lim_m, lim_n;    // kEpiStoreBounded
@@ -583,7 +583,8 @@ __device__ __forceinline__ void gemm_tile(const CUtensorMap *pAh, const CUtensor
   if (args.rowpend && blockIdx.x == 0 && blockIdx.y == 0)
     for (int r = threadIdx.x; r < args.rp_n; r += blockDim.x) args.rowpend[r] = args.rp_val;
   // (warp 2 is idle until the epilogue)
-  if (args.ctl && blockIdx.x == 0 && blockIdx.y == 0 && warp == 2 && lane == 0) finalize_pending(args.ctl);
+  if constexpr (MODE == kEpiSplitScaled)
+    if (args.ctl && blockIdx.x == 0 && blockIdx.y == 0 && warp == 2 && lane == 0) finalize_pending(args.ctl);
 
   if (warp == 0 && lane == 0) {
     // ---- TMA producer ----
@@ -892,8 +893,10 @@ __device__ __forceinline__ void gemm_persist_body(const CUtensorMap *pCh, const 
       decode(t, z, m0, n0);
       const GemmDisk &d = disks[z];
       const int buf = lt & 1;
-      if (d.args.ctl && m0 == 0 && n0 == 0 && warp == 2 && lane == 0) finalize_pending(d.args.ctl);
-      __syncwarp();
+      if constexpr (MODE == kEpiSplitScaled) {
+        if (d.args.ctl && m0 == 0 && n0 == 0 && warp == 2 && lane == 0) finalize_pending(d.args.ctl);
+        __syncwarp();
+      }
       if (!mbar_wait(&acc_full[buf], (lt >> 1) & 1, d.args.status)) {
         abort_flag = 1;
         break;
